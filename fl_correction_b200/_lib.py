@@ -34,7 +34,10 @@ SIGNATURES = {
     "flc_fwd_emission": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
     "flc_bwd_emission": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
     "flc_huber_grad": (_int, [_vp, _vp, _i64, _i64, _i64, _f32, _vp]),
+    "flc_bwd_emission_workspace_bytes": (_sz, [_i64] * 5),
+    "flc_bwd_emission_ws": (_int, [_vp] * 5 + [_i64] * 5 + [_vp, _sz, _vp]),
     "flc_mlem_workspace_bytes": (_sz, [_i64, _i64, _i64, _i64, _i64]),
+    "flc_mlem_workspace_bytes_ex": (_sz, [_i64] * 5),
     "flc_mlem": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _f64, _f64, _i64, _i64, _i64, _i64, _i64,
                         _vp, _sz, _int, _vp]),
     "flc_mlem_static": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _f64, _f64, _i64, _i64, _i64, _i64,
@@ -159,6 +162,21 @@ def workspace(nbytes, device):
     buf = torch.empty(n, dtype=torch.uint8, device=device)
     off = (-buf.data_ptr()) % 256
     return buf[off:off + max(int(nbytes), 1)]
+
+
+def workspace_or_less(nbytes, least, device, limit=None):
+    """A workspace of `nbytes`, or of `least` bytes where the larger one would
+    take more than `limit` (default: a quarter of the device's memory) or
+    cannot be had -- the larger one holds copies that only make the call
+    faster.  Returns it with its size."""
+    if limit is None:
+        limit = torch.cuda.get_device_properties(device).total_memory // 4
+    if least < nbytes <= limit:
+        try:
+            return workspace(nbytes, device), nbytes
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return (workspace(least, device) if least else None), least
 
 
 def ptr_array(tensors):

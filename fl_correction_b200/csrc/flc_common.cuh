@@ -50,7 +50,9 @@ enum TuneKey {
                             // itself only where the lean kernel's image does not fit)
     kTuneXrfBand = 9,       // rows per band of the XRF rotation adjoint (by itself it
                             // bands only slices that do not fit in shared memory)
-    kTuneCount = 10
+    kTuneProjSlices = 10,   // slice-lane kernels where scratch is given: 0 automatic,
+                            // 1 wherever they take the shape, 2 never
+    kTuneCount = 11
 };
 int64_t tune(int key);
 
@@ -62,6 +64,17 @@ int max_smem_optin();
 int smem_per_sm();
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Cluster launches over the angles of a projector kernel (flc_project.cu).
+struct ClusterPlan {
+    int G;      // CTAs per slice or tile (cluster size)
+    int apc;    // angles per CTA
+    size_t smem;
+};
+ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta,
+                         int threads = 512, bool uneven = false);
+int launch_cluster(const void* fn, dim3 grid, int G, size_t smem, cudaStream_t st, void** args,
+                   int threads = 512);
 
 // Bit of the cone `mode` argument that selects the plain separable kernel
 // over the TMA-pipelined one (for parity tests of both).

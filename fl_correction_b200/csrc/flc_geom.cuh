@@ -163,4 +163,32 @@ __device__ __forceinline__ float rot_sample_scipy(const float* __restrict__ img,
     return t.inside ? rot_sample_tap(img, H, W, t) : 0.f;
 }
 
+// Epilogue of a reduced back-projection pixel s of (r, b, h, w):
+//   mode 0: out = s, or max(s, clamp_min) when clamp_min > 0;
+//   mode 1: MLEM update out = max(Cin*s / (sens + beta*huber(Cin)), 0)
+//           (atten_cuda.cpp:331-341), Cin and sens (R,B,H,W) in global memory.
+__device__ __forceinline__ void bwd_epilogue(int mode, float* __restrict__ out,
+                                             const float* __restrict__ Cin,
+                                             const float* __restrict__ sens, float clamp_min,
+                                             float beta, float delta, int r, int b, int B, int H,
+                                             int W, int h, int w, float s) {
+    const int64_t gi = (((int64_t)r * B + b) * H + h) * W + w;
+    if (mode == 0) {
+        out[gi] = clamp_min > 0.f ? fmaxf(s, clamp_min) : s;
+        return;
+    }
+    const float* ci = Cin + ((int64_t)r * B + b) * H * W;
+    const float cp = ci[h * W + w];
+    float den = sens[gi];
+    if (beta > 0.f) {
+        float hg = 0.f;
+        if (h > 0) { float d = cp - ci[(h - 1) * W + w]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
+        if (h + 1 < H) { float d = cp - ci[(h + 1) * W + w]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
+        if (w > 0) { float d = cp - ci[h * W + w - 1]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
+        if (w + 1 < W) { float d = cp - ci[h * W + w + 1]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
+        den = __fadd_rn(den, __fmul_rn(beta, hg));
+    }
+    out[gi] = fmaxf(__fmul_rn(cp, s) / den, 0.f);
+}
+
 }  // namespace flc

@@ -1037,34 +1037,6 @@ __device__ void bwd_splat_angles(const float* __restrict__ atten, const float* _
     fold_frame(cs, sacc, sframe, ncopy, img, pitch, R, H, W);
 }
 
-// Epilogue of a reduced back-projection pixel s of (r, b, h, w):
-//   mode 0: out = s, or max(s, clamp_min) when clamp_min > 0;
-//   mode 1: MLEM update out = max(Cin*s / (sens + beta*huber(Cin)), 0)
-//           (atten_cuda.cpp:331-341), Cin and sens (R,B,H,W) in global memory.
-__device__ __forceinline__ void bwd_epilogue(int mode, float* __restrict__ out,
-                                             const float* __restrict__ Cin,
-                                             const float* __restrict__ sens, float clamp_min,
-                                             float beta, float delta, int r, int b, int B, int H,
-                                             int W, int h, int w, float s) {
-    const int64_t gi = (((int64_t)r * B + b) * H + h) * W + w;
-    if (mode == 0) {
-        out[gi] = clamp_min > 0.f ? fmaxf(s, clamp_min) : s;
-        return;
-    }
-    const float* ci = Cin + ((int64_t)r * B + b) * H * W;
-    const float cp = ci[h * W + w];
-    float den = sens[gi];
-    if (beta > 0.f) {
-        float hg = 0.f;
-        if (h > 0) { float d = cp - ci[(h - 1) * W + w]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
-        if (h + 1 < H) { float d = cp - ci[(h + 1) * W + w]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
-        if (w > 0) { float d = cp - ci[h * W + w - 1]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
-        if (w + 1 < W) { float d = cp - ci[h * W + w + 1]; hg += fabsf(d) <= delta ? d : copysignf(delta, d); }
-        den = __fadd_rn(den, __fmul_rn(beta, hg));
-    }
-    out[gi] = fmaxf(__fmul_rn(cp, s) / den, 0.f);
-}
-
 // Backward with an epilogue: grid (G, B), cluster (G, 1, 1).  CTA g of slice b
 // splats angles [g*apc, (g+1)*apc) (bwd_splat_angles); the cluster then sums
 // its G images over DSMEM in rank order and applies bwd_epilogue.
@@ -1452,11 +1424,7 @@ __global__ void huber_kernel(const float* __restrict__ C, float* __restrict__ gr
 // ---------------------------------------------------------------------------
 // Host-side planning
 // ---------------------------------------------------------------------------
-struct Plan {
-    int G;      // CTAs per slice (cluster size) or angle groups
-    int apc;    // angles per CTA
-    size_t smem;
-};
+}  // namespace
 
 int check_proj_sizes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W) {
     FLC_REQUIRE(A >= 1 && B >= 1 && R >= 1 && H >= 2 && W >= 2,
@@ -1470,9 +1438,11 @@ int check_proj_sizes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W) {
     return FLC_OK;
 }
 
+namespace {
+
 // Clusters of G CTAs of fn (kThreads threads, smem bytes each) that can be
 // resident at once on the current device; 0 if G is not launchable.  Cached.
-int active_clusters(const void* fn, int G, size_t smem, int threads = kThreads) {
+int active_clusters(const void* fn, int G, size_t smem, int threads) {
     struct Entry {
         const void* fn;
         int dev, G;
@@ -1511,13 +1481,17 @@ int active_clusters(const void* fn, int G, size_t smem, int threads = kThreads) 
     return n;
 }
 
+}  // namespace
+
 // Cluster size G (CTAs per slice, each taking ceil(A/G) angles) minimising
 // waves * (angles per CTA + 2): the B clusters run in ceil(B / resident)
 // waves, and each CTA pays about two angles' worth of staging and reduction.
-// The "proj.cluster" knob forces G.
-Plan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta,
-                  int threads = kThreads) {
-    Plan p;
+// `uneven`: the clusters' work differs, so that they even out instead of
+// running in waves: all the work over the resident clusters, and one more
+// cluster's for the tail.  The "proj.cluster" knob forces G.
+ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta, int threads,
+                         bool uneven) {
+    ClusterPlan p;
     p.smem = smem_per_cta;
     int gmax = kMaxCluster < A ? kMaxCluster : (int)A;
     int best_g = 1;
@@ -1528,7 +1502,8 @@ Plan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta,
         for (int G = 1; G <= gmax; ++G) {
             const int n = active_clusters(fn, G, smem_per_cta, threads);
             if (n < 1) continue;
-            const int64_t cost = ceil_div(B, n) * (ceil_div(A, G) + 2);
+            const int64_t item = ceil_div(A, G) + 2;
+            const int64_t cost = uneven ? B * item * 64 / n + item * 64 : ceil_div(B, n) * item;
             if (best < 0 || cost < best) {
                 best = cost;
                 best_g = G;
@@ -1541,7 +1516,7 @@ Plan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta,
 }
 
 int launch_cluster(const void* fn, dim3 grid, int G, size_t smem, cudaStream_t st, void** args,
-                   int threads = kThreads) {
+                   int threads) {
     FLC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     FLC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
@@ -1560,6 +1535,8 @@ int launch_cluster(const void* fn, dim3 grid, int G, size_t smem, cudaStream_t s
     count_launches(1);
     return FLC_OK;
 }
+
+namespace {
 
 size_t tile_floats(int64_t H, int64_t W) { return (size_t)((H * W + 3) & ~3LL); }
 
@@ -1757,7 +1734,7 @@ int bwd2_launch(const float* atten, const float* ratio, const float* em, const f
     const size_t smem = bwd2_smem(R, H, W, ncopy);
     const void* fn = bwd2_kernel_for(R, W);
     const int threads = bwd2_threads(H, W);
-    Plan p = plan_cluster(fn, A, B, smem, threads);
+    ClusterPlan p = plan_cluster(fn, A, B, smem, threads);
     int iA = (int)A, iB = (int)B, iR = (int)R, iH = (int)H, iW = (int)W, apc = p.apc;
     int seg = seg2_length(H, W);
     void* args[] = {(void*)&atten, (void*)&ratio, (void*)&em, (void*)&theta, (void*)&out,
@@ -1813,7 +1790,7 @@ int band_launch(const float* atten, const float* ratio, const float* em, const f
     const int nband = (int)ceil_div(H, hb);
     const size_t smem = band_smem(R, hb, W, ncopy);
     const void* fn = R == 1 ? (const void*)proj_bwd_band_kernel<1> : (const void*)proj_bwd_band_kernel<0>;
-    Plan p = plan_cluster(fn, A, (int64_t)nband * B, smem, kT2);
+    ClusterPlan p = plan_cluster(fn, A, (int64_t)nband * B, smem, kT2);
     int iA = (int)A, iB = (int)B, iR = (int)R, iH = (int)H, iW = (int)W, apc = p.apc, ihb = hb;
     int seg = kSegBand;
     void* args[] = {(void*)&atten, (void*)&ratio, (void*)&em, (void*)&theta, (void*)&out,
@@ -1844,7 +1821,7 @@ int bwd_emission_launch(const float* atten, const float* ratio, const float* em,
     int ncopy = frame_copies([&](int n) { return bwd_smem(R, H, W, stage_tile, n); });
     size_t smem = bwd_smem(R, H, W, stage_tile, ncopy);
     const void* fn = R == 1 ? (const void*)proj_bwd_kernel<1> : (const void*)proj_bwd_kernel<0>;
-    Plan p = plan_cluster(fn, A, B, smem);
+    ClusterPlan p = plan_cluster(fn, A, B, smem);
     int iA = (int)A, iB = (int)B, iR = (int)R, iH = (int)H, iW = (int)W, apc = p.apc;
     int bwd_mode = pick_bwd_mode(H, W), seg = seg_length(H, W);
     void* args[] = {(void*)&atten, (void*)&ratio, (void*)&em, (void*)&theta, (void*)&out,
@@ -1907,7 +1884,7 @@ int mlem_iter_launch(const float* atten, const float* em, const float* theta, co
     int ncopy = frame_copies([&](int n) { return mlem_smem(R, H, W, n); });
     const size_t smem = mlem_smem(R, H, W, ncopy);
     const void* fn = R == 1 ? (const void*)mlem_iter_kernel<1> : (const void*)mlem_iter_kernel<0>;
-    Plan p = plan_cluster(fn, A, B, smem);
+    ClusterPlan p = plan_cluster(fn, A, B, smem);
     int iA = (int)A, iB = (int)B, iR = (int)R, iH = (int)H, iW = (int)W, apc = p.apc;
     int bwd_mode = pick_bwd_mode(H, W), seg = seg_length(H, W);
     void* args[] = {(void*)&atten, (void*)&em, (void*)&theta, (void*)&I, (void*)&sens,

@@ -64,7 +64,7 @@ std::atomic<int64_t> g_tune[kTuneCount];
 const char* const kTuneNames[kTuneCount] = {"proj.cluster", "proj.apc", "cone.variant",
                                             "atten.chunk", "proj.bwd", "cone.test_wait_limit",
                                             "cone.test_skip_load", "proj.legacy", "proj.band",
-                                            "xrf.band"};
+                                            "xrf.band", "proj.slices"};
 }  // namespace
 
 int64_t tune(int key) { return (key >= 0 && key < kTuneCount) ? g_tune[key].load() : 0; }
@@ -108,6 +108,12 @@ int mlem_iter_launch(const float* atten, const float* em, const float* theta, co
                      int64_t R, int64_t H, int64_t W, float beta, float delta, cudaStream_t st,
                      bool* fused, float* ratio_ws);
 void mlem_iter_prepare(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+
+// MLEM on slice-fastest copies (flc_slices.cu).
+size_t mlem_slices_bytes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+int mlem_slices(float* C, const float* atten, const float* em, const float* theta, const float* I,
+                int64_t n_iter, float beta, float delta, int64_t A, int64_t B, int64_t N, void* ws,
+                cudaStream_t st);
 
 namespace {
 
@@ -206,6 +212,14 @@ extern "C" size_t flc_mlem_workspace_bytes(int64_t A, int64_t B, int64_t R, int6
     return mlem_layout(A, B, R, H, W, nullptr, nullptr);
 }
 
+extern "C" size_t flc_mlem_workspace_bytes_ex(int64_t A, int64_t B, int64_t R, int64_t H,
+                                              int64_t W) {
+    if (A < 1 || B < 1 || R < 1 || H < 1 || W < 1) return 0;
+    const size_t base = mlem_layout(A, B, R, H, W, nullptr, nullptr);
+    const size_t ex = mlem_slices_bytes(A, B, R, H, W);
+    return ex > base ? ex : base;
+}
+
 extern "C" int flc_mlem(float* C, const float* atten, const float* em, const float* theta,
                         const float* I, int64_t n_iter, double beta, double delta, int64_t A,
                         int64_t B, int64_t R, int64_t H, int64_t W, void* workspace,
@@ -226,6 +240,12 @@ extern "C" int flc_mlem(float* C, const float* atten, const float* em, const flo
         return FLC_ERR_WORKSPACE;
     }
     cudaStream_t st = as_stream(stream);
+    if (n_iter > 0) {
+        const size_t ex = mlem_slices_bytes(A, B, R, H, W);
+        if (ex > 0 && workspace_bytes >= (ex > need ? ex : need))
+            return mlem_slices(C, atten, em, theta, I, n_iter, (float)beta, (float)delta, A, B, H,
+                               workspace, st);
+    }
     MlemBufs m;
     mlem_layout(A, B, R, H, W, (char*)workspace, &m);
     // sens = max(P^T 1, 1e-6)   (atten_cuda.cpp:308-314)

@@ -85,6 +85,6 @@ extern "C" int flc_mlem_static(float* C, const float* atten, const float* em, co
     }
     void* ws = nullptr;
     FLC_TRY(static_scratch(&ws));
-    return flc_mlem(C, atten, em, theta, I, n_iter, beta, delta, A, B, R, H, W, ws,
-                    kStaticScratchBytes, 0, stream);
+    return flc_mlem(C, atten, em, theta, I, n_iter, beta, delta, A, B, R, H, W, ws, need, 0,
+                    stream);
 }

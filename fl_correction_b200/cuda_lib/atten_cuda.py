@@ -117,8 +117,10 @@ def backward_emission_batch(atten, ratio, em_cs, theta):
     R = em_cs.shape[1]
     out = torch.empty((R, B, H, W), dtype=atten.dtype, device=atten.device)
     with torch.cuda.device(atten.device):
-        _lib.call("flc_bwd_emission", _lib.ptr(atten), _lib.ptr(ratio), _lib.ptr(em_cs),
-                  _lib.ptr(theta), _lib.ptr(out), A, B, R, H, W, _lib.stream())
+        nb = _lib.query("flc_bwd_emission_workspace_bytes", A, B, R, H, W)
+        ws, nb = _lib.workspace_or_less(nb, 0, atten.device) if nb else (None, 0)
+        _lib.call("flc_bwd_emission_ws", _lib.ptr(atten), _lib.ptr(ratio), _lib.ptr(em_cs),
+                  _lib.ptr(theta), _lib.ptr(out), A, B, R, H, W, _lib.ptr(ws), nb, _lib.stream())
     return out
 
 
@@ -168,9 +170,10 @@ def mlem_cuda_batch(C_init, atten, em_cs, theta, I, n_iter, beta=1e-3, delta=0.0
     R = C_init.shape[0]
     C = C_init.clone(memory_format=torch.contiguous_format)
     atten, em_cs, theta, I = _c(atten), _c(em_cs), _c(theta), _c(I)
-    ws_bytes = _lib.query("flc_mlem_workspace_bytes", A, B, R, H, W)
-    ws = _lib.workspace(ws_bytes, atten.device)
     with torch.cuda.device(atten.device):
+        ws, ws_bytes = _lib.workspace_or_less(
+            _lib.query("flc_mlem_workspace_bytes_ex", A, B, R, H, W),
+            _lib.query("flc_mlem_workspace_bytes", A, B, R, H, W), atten.device)
         _lib.call("flc_mlem", _lib.ptr(C), _lib.ptr(atten), _lib.ptr(em_cs), _lib.ptr(theta),
                   _lib.ptr(I), int(n_iter), float(beta), float(delta), A, B, R, H, W,
                   _lib.ptr(ws), ws_bytes, 1, _lib.stream())

@@ -94,8 +94,15 @@ class CorrectedMLEM:
         ws, _, _ = atten_workspace_bytes(self.n_ch, S, H, W, A, self.L, chunk, self.mask_uv[2])
         self.chunk = chunk
         self.ws_atten = _lib.workspace(ws, dev)
-        self.ws_mlem_bytes = _lib.query("flc_mlem_workspace_bytes", A, S, 1, H, W)
-        self.ws_mlem = _lib.workspace(self.ws_mlem_bytes, dev)
+        n_ws = self.L if self.concurrent else 1
+        least = _lib.query("flc_mlem_workspace_bytes", A, S, 1, H, W)
+        # the copies of the slice-lane MLEM, where a quarter of the free memory
+        # holds those of every element
+        free = (torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev)
+                - torch.cuda.memory_allocated(dev))
+        with torch.cuda.device(dev):
+            most = least if multi else _lib.query("flc_mlem_workspace_bytes_ex", A, S, 1, H, W)
+        self.ws_mlem, self.ws_mlem_bytes = _lib.workspace_or_less(most, least, dev, free // (4 * n_ws))
         self._elem = None
         if self.concurrent and self.L > 1:
             # one stream and one MLEM workspace per element

@@ -75,6 +75,9 @@ FLC_API uint64_t flc_launch_count(void);
  *                   where a slice image does not fit in shared memory) at every size
  *   "xrf.band"      rows per band of the XRF rotation adjoint (automatic: the whole
  *                   slice, or the fewest even bands that fit in shared memory)
+ *   "proj.slices"   the slice-lane kernels of flc_mlem and flc_bwd_emission_ws (square
+ *                   slices, where scratch is given): 1 wherever they take the shape, 2
+ *                   never; automatic: from 16 slices on
  * Test hooks of the direct cone's bounded waits (for failure-path tests):
  *   "cone.test_wait_limit"  polls before a TMA-plane wait gives up (default 2^26)
  *   "cone.test_skip_load"   k > 0: the load of the k-th staged plane of every
@@ -148,6 +151,18 @@ FLC_API int flc_bwd_emission(const float* atten, const float* ratio, const float
                      const float* theta, float* out, int64_t A, int64_t B, int64_t R,
                      int64_t H, int64_t W, void* stream);
 
+/* flc_bwd_emission with caller scratch, for volumes: `workspace` (256-byte
+ * aligned) of flc_bwd_emission_workspace_bytes(...) bytes lets the backward
+ * run on slice-fastest copies of a part of the angles at a time (about 512
+ * MB), with the slices as lanes.  Where that is 0 (few slices, slices that are
+ * not square), or workspace is NULL or smaller, the call is flc_bwd_emission. */
+FLC_API size_t flc_bwd_emission_workspace_bytes(int64_t A, int64_t B, int64_t R, int64_t H,
+                                                int64_t W);
+FLC_API int flc_bwd_emission_ws(const float* atten, const float* ratio, const float* em,
+                        const float* theta, float* out, int64_t A, int64_t B, int64_t R,
+                        int64_t H, int64_t W, void* workspace, size_t workspace_bytes,
+                        void* stream);
+
 /* Huber gradient over the four in-plane neighbours of each pixel of
  * C (RB, H, W).  Replaces huber_grad[_batch]
  * (atten_cuda.cpp:218-238; atten_cuda_kernel.cu:495-616). */
@@ -161,9 +176,14 @@ FLC_API int flc_huber_grad(const float* C, float* grad, int64_t RB, int64_t H, i
  * copies C_init first, as the reference's clone does).  I is (A,B,W).
  * The caller provides `workspace` of at least flc_mlem_workspace_bytes(...)
  * bytes (256-byte aligned).  With use_graph != 0 the iteration is captured
- * once into a CUDA graph and replayed n_iter times.
+ * once into a CUDA graph and replayed n_iter times.  A workspace of
+ * flc_mlem_workspace_bytes_ex(...) bytes lets volumes of one reference run on
+ * slice-fastest copies of the attenuation, the projections and the images,
+ * with the slices as lanes (it holds a copy of the attenuation; where that
+ * form does not take the call, it is flc_mlem_workspace_bytes(...)).
  * --------------------------------------------------------------------- */
 FLC_API size_t flc_mlem_workspace_bytes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+FLC_API size_t flc_mlem_workspace_bytes_ex(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
 FLC_API int flc_mlem(float* C, const float* atten, const float* em, const float* theta,
              const float* I, int64_t n_iter, double beta, double delta,
              int64_t A, int64_t B, int64_t R, int64_t H, int64_t W,
