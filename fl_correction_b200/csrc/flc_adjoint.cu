@@ -39,7 +39,7 @@ int cone_launch_ws(const float* mu, const float* U, const float* Vw, float* out,
                    int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
                    int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, void* ws,
                    size_t ws_bytes, cudaStream_t st);
-size_t cone_fft_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
+size_t cone_spec_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
                          int64_t My, int mode);
 size_t frac4_bytes(int64_t n_ch, int64_t S, int64_t H, int64_t W);
 int frac_interleave_launch(const float* frac, float4* frac4, int64_t n_ch, int64_t S, int64_t H,
@@ -529,7 +529,7 @@ extern "C" size_t flc_xrf_workspace_bytes_ex(int64_t n_ch, int64_t S, int64_t H,
     const int64_t c = xrf_chunk(S, H, W, A, L, chunk);
     // cone frame (Z = S, X = W, Y = H); the beam-layout modes need the most
     return xrf_ws_bytes(S, H, W, A, L, chunk) + frac4_bytes(n_ch, S, H, W) +
-           cone_fft_ws_bytes(c * L, S, W, H, Mz, Mx, My, 2);
+           cone_spec_ws_bytes(c * L, S, W, H, Mz, Mx, My, 2);
 }
 
 extern "C" int flc_xrf_project(const float* frac, const float* theta, const float* coef_x,

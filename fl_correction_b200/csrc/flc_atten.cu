@@ -515,8 +515,12 @@ int cone_tma_launch(const float* mu, const float* U, const float* Vw, float* out
                     int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, cudaStream_t st);
 
 // Spectral form (flc_cone_fft.cu).
-size_t cone_fft_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
+size_t cone_spec_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
                          int64_t My, int mode);
+int cone_line_launch(const float* mu, const float* U, const float* Vw, float* out, int64_t Vn,
+                     int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
+                     int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, void* workspace,
+                     size_t ws_bytes, cudaStream_t st);
 int cone_fft_launch(const float* mu, const float* U, const float* Vw, float* out, int64_t Vn,
                     int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
                     int L, int a_base, int64_t out_a_stride, int64_t out_l_stride,
@@ -551,17 +555,21 @@ int cone_sep_launch(const float* mu, const float* U, const float* Vw, float* out
     return check_launch("cone_sep_kernel");
 }
 
-// Cone path sum with scratch for the spectral form: the spectral kernels run
-// when the "cone.variant" knob allows them (0 automatic, 4 spectral, 5
-// spectral with split plane transforms) and the shape and scratch fit;
-// otherwise cone_sep_launch.
+// Cone path sum with scratch for the spectral forms: the line form where a plane
+// of (x, z) lines fits in shared memory (128^3, 96^3, 64 x 256^2), else the plane
+// form (split where a padded plane does not fit), when the "cone.variant" knob
+// allows them (0 automatic, 4 spectral, 5 the split plane form) and the scratch
+// is there; otherwise cone_sep_launch.
 int cone_launch_ws(const float* mu, const float* U, const float* Vw, float* out, int64_t Vn,
                    int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
                    int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, void* ws,
                    size_t ws_bytes, cudaStream_t st) {
     const int64_t var = tune(kTuneConeVariant);
     if (ws && (var == 0 || var == 4 || var == 5)) {
-        int r = cone_fft_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
+        int r = cone_line_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
+                                 out_a_stride, out_l_stride, ws, ws_bytes, st);
+        if (r == FLC_ERR_UNSUPPORTED)
+            r = cone_fft_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
                                 out_a_stride, out_l_stride, ws, ws_bytes, st);
         if (r != FLC_ERR_UNSUPPORTED) return r;
         clear_error();
@@ -769,7 +777,7 @@ extern "C" int flc_cone_atten_separable(const float* mu, const float* u, const f
 extern "C" size_t flc_cone_atten_workspace_bytes(int64_t K, int64_t Z, int64_t X, int64_t Y,
                                                  int64_t Mz, int64_t Mx, int64_t My) {
     if (K < 1 || Z < 1 || X < 1 || Y < 1 || Mz < 1 || Mx < 1 || My < 1) return 0;
-    return cone_fft_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
+    return cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
 }
 
 extern "C" int flc_cone_atten_separable_ws(const float* mu, const float* u, const float* v,
@@ -812,7 +820,7 @@ extern "C" int flc_cone_atten(const float* mu, const float* mask, float* out, in
         // where the shape takes it
         float* dbuf = nullptr;
         const size_t fbytes = align256(sizeof(float) * (U.size() + V.size()));
-        const size_t fft_bytes = cone_fft_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
+        const size_t fft_bytes = cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
         const size_t bytes = fbytes + (fft_bytes ? fft_bytes + 256 : 0);
         FLC_TRY_CUDA(cudaMallocAsync((void**)&dbuf, bytes, st));
         int s = FLC_OK;
@@ -1017,7 +1025,7 @@ extern "C" size_t flc_cone_fft_workspace_bytes(int64_t n_vol, int64_t S, int64_t
                                                int64_t Mz, int64_t Mx, int64_t My) {
     if (n_vol < 1 || S < 1 || H < 1 || W < 1 || Mz < 1 || Mx < 1 || My < 1) return 0;
     // cone frame (Z = S, X = W, Y = H), beam-layout output
-    return cone_fft_ws_bytes(n_vol, S, W, H, Mz, Mx, My, 2);
+    return cone_spec_ws_bytes(n_vol, S, W, H, Mz, Mx, My, 2);
 }
 
 extern "C" int flc_cone_atten_apply_ws(const float* mu_ref, const float* u, const float* v,

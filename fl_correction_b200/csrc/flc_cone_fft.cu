@@ -19,6 +19,9 @@
 // rounded from FP64); the result agrees with the FP64 oracle to ~1e-6 of
 // its largest value.
 //
+// This plane form runs where the line form (flc_cone_line.cu) does not take the
+// shape, its scratch is not there, or the "cone.variant" knob is 5.
+//
 // Kernels, in launch order:
 //   fft_filter_kernel : G (Mx x Nz x Nyh) and the twiddle tables, FP64 -> FP32
 //   fft_fwd_kernel    : one CTA per (volume, plane): rows (two real rows per

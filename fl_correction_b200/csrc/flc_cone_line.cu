@@ -1,0 +1,979 @@
+// Spectral cone path sum with line transforms in registers (sm_100a).
+//
+// The algorithm is that of flc_cone_fft.cu -- the depth sum of 2-D correlations
+// as pointwise products of (z, y) spectra -- taken one axis further: along the
+// depth, R_x = sum_d G_d P_{x+d} is a correlation too, so with the depth padded
+// to Nx >= X + min(Mx, X) - 1 it is one product per frequency,
+//   Rhat(kx) = Ghat(kx) Phat(kx),  Ghat(kx) = sum_d G_d e^{+2 pi i kx d / Nx},
+// 22 instead of 66 kFLOP per frequency of a 128^3 volume.
+//
+// Two volumes travel together as the real and imaginary part of one complex
+// volume (the kernel is real, so the path sum acts on both alike): there are no
+// half spectra to unpack.  Every transform has a length N = R1 R2 and runs in
+// two steps of R1- and R2-point DFTs, one line segment per thread in registers,
+// in place: element n = R2 n1 + n2 becomes A(k1, n2) at R2 k1 + n2, that
+// becomes X(k1 + R1 k2) at R2 k1 + k2.  The spectra stay in that order (the
+// filter is made in it), and the inverse takes the same steps back.
+//
+//   line_roots, line_filter : twiddles, the mask's line spectra, Ghat
+//   line_rows   : mu -> S[ky][x][z]; 32 rows of one plane x per CTA, transforms
+//                 along y
+//   line_mid    : per (ky, pair of volumes), the whole (x, z) plane in shared
+//                 memory: transform along z; along x, times Ghat, back; back
+//                 along z; S[ky][z][x] over the same memory
+//   line_out    : transforms back along y, 32 x of one slice z per CTA, and
+//                 writes exp(-res) into the beam layout (x is its fastest axis,
+//                 so no transpose is left) or res into the reference layout
+//
+// 30 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.13, middle 0.59, out 0.23,
+// filter 0.04 ms, against 1.83 ms in five kernels of the plane form.  Rows and out
+// move the bytes they must at about half the copy rate; the middle is bound by the
+// latency of its steps (one CTA of 16 warps per SM: the plane takes 148 KB).  Teams
+// of 128 / 256 / 512 threads there: 0.60 / 0.57 / 0.66 ms; strides known at run time
+// only: 0.66; the spectra in batches small enough for L2 (40, 80 MB): 0.74, 0.71.
+
+#include <algorithm>
+
+#include "flc_common.cuh"
+
+namespace flc {
+
+size_t cone_fft_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
+                         int64_t My, int mode);
+
+namespace {
+
+typedef unsigned long long c32;   // complex FP32 in a register pair
+
+__device__ __forceinline__ c32 mk(float a, float b) {
+    c32 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void un(c32 r, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+// PK: one paired instruction instead of two scalar ones.  The paired form costs
+// registers; it is the faster one in line_mid (0.60 against 0.63 ms for 30 volumes
+// of 128^3), the scalar one in line_out (0.28 against 0.23 ms).
+template <bool PK>
+__device__ __forceinline__ c32 cadd(c32 a, c32 b) {
+    if constexpr (PK) {
+        c32 d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    } else {
+        float x, y, u, v;
+        un(a, x, y);
+        un(b, u, v);
+        return mk(x + u, y + v);
+    }
+}
+template <bool PK>
+__device__ __forceinline__ c32 csub(c32 a, c32 b) {
+    if constexpr (PK) {
+        c32 d;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(mk(-1.f, -1.f)), "l"(a));
+        return d;
+    } else {
+        float x, y, u, v;
+        un(a, x, y);
+        un(b, u, v);
+        return mk(x - u, y - v);
+    }
+}
+__device__ __forceinline__ c32 cmul2(c32 a, c32 b) {   // halves apart
+    c32 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ c32 cfma2(c32 a, c32 b, c32 c) {
+    c32 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// z (c + i s): four scalar instructions (paired ones would need the halves swapped)
+__device__ __forceinline__ c32 cturn(c32 z, float c, float s) {
+    float x, y;
+    un(z, x, y);
+    return mk(fmaf(c, x, -s * y), fmaf(c, y, s * x));
+}
+// z * i^{SG}
+template <int SG>
+__device__ __forceinline__ c32 crot(c32 z) {
+    float x, y;
+    un(z, x, y);
+    return SG > 0 ? mk(-y, x) : mk(y, -x);
+}
+
+// cos and sin of 2 pi m / n at compile time, by their power series.
+constexpr double series(double x, bool sine) {
+    double t = sine ? x : 1.0, sum = t;
+    for (int k = sine ? 2 : 1; k < 40; k += 2) {
+        t *= -x * x / (double)(k * (k + 1));
+        sum += t;
+    }
+    return sum;
+}
+constexpr double kTwoPi = 6.283185307179586476925286766559;
+constexpr double angle(int m, int n) {
+    m %= n;
+    if (2 * m > n) m -= n;
+    return kTwoPi * (double)m / (double)n;
+}
+constexpr float cos_of(int m, int n) { return (float)series(angle(m, n), false); }
+constexpr float sin_of(int m, int n) { return (float)series(angle(m, n), true); }
+
+// v[k] = sum_n v[n] e^{SG 2 pi i n k / R}, in place, natural order.
+template <int R, int SG, bool PK>
+__device__ __forceinline__ void dft(c32 (&v)[R]);
+
+template <int P, int Q, int SG, bool PK>
+__device__ __forceinline__ void dft_pq(c32 (&v)[P * Q]) {
+    constexpr int R = P * Q;
+    c32 y[Q][P];
+#pragma unroll
+    for (int n2 = 0; n2 < Q; ++n2) {
+        c32 t[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) t[n1] = v[Q * n1 + n2];
+        dft<P, SG, PK>(t);
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) {
+            const int m = n2 * k1;
+            y[n2][k1] = m == 0 ? t[k1]
+                      : 4 * m == R ? crot<SG>(t[k1])
+                                   : cturn(t[k1], cos_of(m, R), SG * sin_of(m, R));
+        }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) {
+        c32 u[Q];
+#pragma unroll
+        for (int n2 = 0; n2 < Q; ++n2) u[n2] = y[n2][k1];
+        dft<Q, SG, PK>(u);
+#pragma unroll
+        for (int k2 = 0; k2 < Q; ++k2) v[k1 + P * k2] = u[k2];
+    }
+}
+
+template <int R, int SG, bool PK>
+__device__ __forceinline__ void dft(c32 (&v)[R]) {
+    if constexpr (R == 2) {
+        const c32 a = v[0], b = v[1];
+        v[0] = cadd<PK>(a, b);
+        v[1] = csub<PK>(a, b);
+    } else if constexpr (R == 3) {
+        const c32 a = cadd<PK>(v[1], v[2]);
+        const c32 t = cfma2(mk(-0.5f, -0.5f), a, v[0]);
+        const c32 d = csub<PK>(v[1], v[2]);
+        constexpr float s3 = 0.866025403784438647f;
+        const c32 u = cmul2(mk(s3, s3), crot<SG>(d));
+        v[0] = cadd<PK>(v[0], a);
+        v[1] = cadd<PK>(t, u);
+        v[2] = csub<PK>(t, u);
+    } else if constexpr (R == 4) {
+        const c32 s02 = cadd<PK>(v[0], v[2]), d02 = csub<PK>(v[0], v[2]);
+        const c32 s13 = cadd<PK>(v[1], v[3]), w13 = crot<SG>(csub<PK>(v[1], v[3]));
+        v[0] = cadd<PK>(s02, s13);
+        v[2] = csub<PK>(s02, s13);
+        v[1] = cadd<PK>(d02, w13);
+        v[3] = csub<PK>(d02, w13);
+    } else if constexpr (R == 5) {
+        constexpr float c1 = 0.309016994374947424f, c2 = -0.809016994374947424f;
+        constexpr float s1 = 0.951056516295153572f, s2 = 0.587785252292473129f;
+        const c32 a1 = cadd<PK>(v[1], v[4]), b1 = crot<SG>(csub<PK>(v[1], v[4]));
+        const c32 a2 = cadd<PK>(v[2], v[3]), b2 = crot<SG>(csub<PK>(v[2], v[3]));
+        const c32 t1 = cfma2(mk(c2, c2), a2, cfma2(mk(c1, c1), a1, v[0]));
+        const c32 t2 = cfma2(mk(c1, c1), a2, cfma2(mk(c2, c2), a1, v[0]));
+        const c32 u1 = cfma2(mk(s2, s2), b2, cmul2(mk(s1, s1), b1));
+        const c32 u2 = cfma2(mk(-s1, -s1), b2, cmul2(mk(s2, s2), b1));
+        v[0] = cadd<PK>(v[0], cadd<PK>(a1, a2));
+        v[1] = cadd<PK>(t1, u1);
+        v[4] = csub<PK>(t1, u1);
+        v[2] = cadd<PK>(t2, u2);
+        v[3] = csub<PK>(t2, u2);
+    } else if constexpr (R == 6) {
+        dft_pq<2, 3, SG, PK>(v);
+    } else if constexpr (R == 8) {
+        dft_pq<2, 4, SG, PK>(v);
+    } else if constexpr (R == 9) {
+        dft_pq<3, 3, SG, PK>(v);
+    } else if constexpr (R == 10) {
+        dft_pq<2, 5, SG, PK>(v);
+    } else if constexpr (R == 12) {
+        dft_pq<3, 4, SG, PK>(v);
+    } else if constexpr (R == 16) {
+        dft_pq<4, 4, SG, PK>(v);
+    } else if constexpr (R == 18) {
+        dft_pq<2, 9, SG, PK>(v);
+    } else if constexpr (R == 20) {
+        dft_pq<4, 5, SG, PK>(v);
+    } else {
+        static_assert(R == 32, "radix");
+        dft_pq<4, 8, SG, PK>(v);
+    }
+}
+
+// v[k] *= e^{SG 2 pi i m k / N}, k = 1 .. R-1; tw[j] = e^{-2 pi i j / N}.
+template <int R, int SG>
+__device__ __forceinline__ void twiddle(c32 (&v)[R], const float2* tw, int m) {
+#pragma unroll
+    for (int k = 1; k < R; ++k) {
+        const float2 t = tw[m * k];
+        v[k] = cturn(v[k], t.x, SG < 0 ? t.y : -t.y);
+    }
+}
+
+struct Len {
+    int n, r1, r2, id;
+};
+
+struct LineGeom {
+    int Z, X, Y, Mz, Mx, My;
+    Len z, x, y;
+    int team;       // line_mid: threads of a team,
+    int G;          // and the kz lines it takes per depth pass
+};
+
+// Transform lengths R1 R2, as F(index, R1, R2), shortest first; the longest ones
+// for the depth only.  The steps are compiled for each, so that strides and
+// pitches are immediates.
+#define FLC_LENS(F)                                                                         \
+    F(0, 4, 4) F(1, 6, 4) F(2, 8, 4) F(3, 8, 5) F(4, 8, 6) F(5, 9, 6) F(6, 8, 8) F(7, 9, 8) \
+    F(8, 10, 8) F(9, 10, 9) F(10, 12, 8) F(11, 12, 9) F(12, 12, 10) F(13, 16, 8)            \
+    F(14, 12, 12) F(15, 16, 10) F(16, 18, 10) F(17, 16, 12) F(18, 18, 12) F(19, 20, 12)     \
+    F(20, 16, 16) F(21, 18, 16) F(22, 20, 16) F(23, 20, 20)
+#define FLC_LENS_X(F)                                                                       \
+    F(24, 32, 16) F(25, 32, 20)
+
+#define FLC_CASE(i, A, B) case i: CALL(A, B); break;
+#define FLC_LEN(l) switch ((l).id) { FLC_LENS(FLC_CASE) }
+#define FLC_LEN_X(l) switch ((l).id) { FLC_LENS(FLC_CASE) FLC_LENS_X(FLC_CASE) }
+
+constexpr int kRowsT = 256;      // threads of line_rows / line_out
+constexpr int kLines = 32;       // lines per CTA of line_rows / line_out
+constexpr int kMidT = 512;
+
+// floor(a / b) for 0 <= a < 2^22 from b's reciprocal.
+__device__ __forceinline__ int div_small(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
+
+// ---------------------------------------------------------------------------
+// Twiddles T[m] = e^{-2 pi i m / N} of the three lengths, and the line spectra
+// Uf_d(kz) = sum_dz u[d][dz] e^{+2 pi i kz (dz - hz) / Nz} (Vf likewise) in FP64,
+// in the transforms' order.  Grid Mx + 1: block d < Mx its spectra, block Mx the
+// twiddles.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+line_roots_kernel(const float* __restrict__ U, const float* __restrict__ V, double2* __restrict__ Uf,
+                  double2* __restrict__ Vf, float2* __restrict__ Tz, float2* __restrict__ Tx,
+                  float2* __restrict__ Ty, LineGeom g) {
+    extern __shared__ double2 root[];      // e^{2 pi i m / N} of z, then y
+    const int d = blockIdx.x, Nz = g.z.n, Ny = g.y.n;
+    if (d == g.Mx) {
+        for (int m = threadIdx.x; m < Nz + g.x.n + Ny; m += blockDim.x) {
+            const int n = m < Nz ? Nz : m < Nz + g.x.n ? g.x.n : Ny;
+            const int mm = m < Nz ? m : m < Nz + g.x.n ? m - Nz : m - Nz - g.x.n;
+            float2* T = m < Nz ? Tz : m < Nz + g.x.n ? Tx : Ty;
+            double s, c;
+            sincospi(-2.0 * (double)mm / (double)n, &s, &c);
+            T[mm] = make_float2((float)c, (float)s);
+        }
+        return;
+    }
+    for (int m = threadIdx.x; m < Nz + Ny; m += blockDim.x) {
+        double s, c;
+        sincospi(m < Nz ? 2.0 * (double)m / (double)Nz : 2.0 * (double)(m - Nz) / (double)Ny, &s, &c);
+        root[m] = make_double2(c, s);
+    }
+    __syncthreads();
+    const int hz = g.Mz / 2, hy = g.My / 2;
+    for (int p = threadIdx.x; p < Nz + Ny; p += blockDim.x) {
+        const bool zk = p < Nz;
+        const Len l = zk ? g.z : g.y;
+        const int pos = zk ? p : p - Nz, n = l.n, M = zk ? g.Mz : g.My, h = zk ? hz : hy;
+        const int k = pos / l.r2 + l.r1 * (pos % l.r2);      // frequency at this place
+        const float* w = zk ? U + (int64_t)d * g.Mz : V + (int64_t)d * g.My;
+        const double2* rt = zk ? root : root + Nz;
+        int m = (int)(((int64_t)k * (n - h % n)) % n);
+        double re = 0.0, im = 0.0;
+        for (int t = 0; t < M; ++t) {
+            const double wt = (double)__ldg(w + t);
+            re += wt * rt[m].x;
+            im += wt * rt[m].y;
+            m += k;
+            if (m >= n) m -= n;
+        }
+        (zk ? Uf : Vf)[(int64_t)d * n + pos] = make_double2(re, im);
+    }
+}
+
+// Ghat[ky][kx][kz] (all in the transforms' order): G_d = Uf_d(kz) Vf_d(ky), rounded
+// from FP64, transformed along d with the + sign.  Grid (Ny, ceil(Nz / 16)).
+constexpr int kFilterG = 16;
+
+template <int R, int R2>
+__device__ __forceinline__ void filter_a(const double2* Uf, const double2* Vf, c32* xb, const float2* tw,
+                                         const LineGeom& g, int ky, int kz0, int nk) {
+    constexpr int r2 = R2, P = R * R2 + 1;
+    const int D = min(g.Mx, g.X);
+    for (int i = threadIdx.x; i < kFilterG * r2; i += blockDim.x) {
+        const int kl = i % kFilterG, n2 = i / kFilterG;
+        if (kl >= nk) continue;
+        c32 v[R];
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) {
+            const int d = r2 * n1 + n2;
+            v[n1] = mk(0.f, 0.f);
+            if (d < D) {
+                const double2 a = Uf[(int64_t)d * g.z.n + kz0 + kl], b = Vf[(int64_t)d * g.y.n + ky];
+                v[n1] = mk((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
+            }
+        }
+        dft<R, 1, false>(v);
+        twiddle<R, 1>(v, tw, n2);
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) xb[kl * P + r2 * k1 + n2] = v[k1];
+    }
+}
+
+template <int R1, int R>
+__device__ __forceinline__ void filter_b(const c32* xb, c32* Gh, const LineGeom& g, int kz0, int nk) {
+    constexpr int P = R1 * R + 1;
+    for (int i = threadIdx.x; i < kFilterG * R1; i += blockDim.x) {
+        const int kl = i % kFilterG, k1 = i / kFilterG;
+        if (kl >= nk) continue;
+        c32 v[R];
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) v[n2] = xb[kl * P + R * k1 + n2];
+        dft<R, 1, false>(v);
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) Gh[(int64_t)(R * k1 + k2) * g.z.n + kz0 + kl] = v[k2];
+    }
+}
+
+__global__ void __launch_bounds__(256)
+line_filter_kernel(const double2* __restrict__ Uf, const double2* __restrict__ Vf,
+                   const float2* __restrict__ Tx, c32* __restrict__ Gh, LineGeom g) {
+    extern __shared__ __align__(16) c32 sf[];
+    c32* xb = sf;                                                   // [16][Nx + 1]
+    float2* tw = reinterpret_cast<float2*>(xb + kFilterG * (g.x.n + 1));
+    for (int m = threadIdx.x; m < g.x.n; m += blockDim.x) tw[m] = Tx[m];
+    __syncthreads();
+    const int ky = blockIdx.x, kz0 = blockIdx.y * kFilterG, nk = min(kFilterG, g.z.n - kz0);
+#define CALL(A, B) filter_a<A, B>(Uf, Vf, xb, tw, g, ky, kz0, nk)
+    FLC_LEN_X(g.x)
+#undef CALL
+    __syncthreads();
+    c32* Gk = Gh + (int64_t)ky * g.x.n * g.z.n;
+#define CALL(A, B) filter_b<A, B>(xb, Gk, g, kz0, nk)
+    FLC_LEN_X(g.x)
+#undef CALL
+}
+
+// ---------------------------------------------------------------------------
+// Rows forward: grid (ceil(Z / 32), X, pairs).  Volume 2p is the real part,
+// 2p + 1 (if it exists) the imaginary part.
+// ---------------------------------------------------------------------------
+template <int R, int R2>
+__device__ __forceinline__ void rows_a(const float* ma, const float* mb, c32* sm, const float2* tw,
+                                       const LineGeom& g, int nl) {
+    constexpr int r2 = R2, P = R * R2 + 1;
+    const int64_t zs = (int64_t)g.X * g.Y;
+    for (int i = threadIdx.x; i < nl * r2; i += kRowsT) {
+        const int l = i / r2, n2 = i - l * r2;
+        float a[R], b[R];
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) {
+            const int y = r2 * n1 + n2;
+            a[n1] = y < g.Y ? __ldg(ma + l * zs + y) : 0.f;
+            b[n1] = y < g.Y && mb ? __ldg(mb + l * zs + y) : 0.f;
+        }
+        c32 v[R];
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) v[n1] = mk(a[n1], b[n1]);
+        dft<R, -1, false>(v);
+        twiddle<R, -1>(v, tw, n2);
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) sm[l * P + r2 * k1 + n2] = v[k1];
+    }
+}
+
+template <int R1, int R>
+__device__ __forceinline__ void rows_b(const c32* sm, c32* S, const LineGeom& g, int nl) {
+    constexpr int P = R1 * R + 1;
+    const int64_t ks = (int64_t)g.X * g.Z;
+    const int l = threadIdx.x & 31;
+    if (l >= nl) return;
+    for (int k1 = threadIdx.x >> 5; k1 < R1; k1 += kRowsT / 32) {
+        c32 v[R];
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) v[n2] = sm[l * P + R * k1 + n2];
+        dft<R, -1, false>(v);
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) S[(R * k1 + k2) * ks + l] = v[k2];
+    }
+}
+
+__global__ void __launch_bounds__(kRowsT, 3)
+line_rows_kernel(const float* __restrict__ mu, const float2* __restrict__ Ty, c32* __restrict__ S,
+                 LineGeom g, int Vn) {
+    extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
+    float2* tw = reinterpret_cast<float2*>(sm + kLines * (g.y.n + 1));
+    for (int m = threadIdx.x; m < g.y.n; m += kRowsT) tw[m] = Ty[m];
+    __syncthreads();
+    const int z0 = blockIdx.x * kLines, x = blockIdx.y, p = blockIdx.z;
+    const int nl = min(kLines, g.Z - z0);
+    const int64_t vol = (int64_t)g.Z * g.X * g.Y;
+    const float* ma = mu + 2 * p * vol + ((int64_t)z0 * g.X + x) * g.Y;
+    const float* mb = 2 * p + 1 < Vn ? ma + vol : nullptr;
+#define CALL(A, B) rows_a<A, B>(ma, mb, sm, tw, g, nl)
+    FLC_LEN(g.y)
+#undef CALL
+    __syncthreads();
+    c32* Sp = S + ((int64_t)p * g.y.n * g.X + x) * g.Z + z0;
+#define CALL(A, B) rows_b<A, B>(sm, Sp, g, nl)
+    FLC_LEN(g.y)
+#undef CALL
+}
+
+// ---------------------------------------------------------------------------
+// Middle: grid (Ny, pairs), one CTA per SM with the (x, z) plane of one ky.  The
+// threads work in teams, each on its own x lines (transforms along z) and its own
+// kz lines (along the depth, in a buffer of its own), with barriers of the team
+// only: while one waits for Ghat or at a barrier, the others run.
+// ---------------------------------------------------------------------------
+struct Team {
+    int t, n, id;     // thread in the team, threads, team
+    int x0, x1;       // its x lines
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "r"(n) : "memory");
+    }
+};
+
+// z step 1 (adjacent threads along x: the pitch Nz + 1 is odd or spreads over the
+// banks, and a warp reads one twiddle); samples z >= Z are zero.
+template <int R, int R2>
+__device__ __forceinline__ void mid_za(c32* pl, const float2* tw, const LineGeom& g, const Team& tm) {
+    constexpr int r2 = R2, P = R * R2 + 1;
+    const int nx = tm.x1 - tm.x0;
+    const float rX = 1.f / (float)nx;
+    for (int i = tm.t; i < nx * r2; i += tm.n) {
+        const int n2 = div_small(i, rX), x = tm.x0 + i - n2 * nx;
+        c32* row = pl + x * P + n2;
+        c32 v[R];
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) v[n1] = r2 * n1 + n2 < g.Z ? row[r2 * n1] : 0ull;
+        dft<R, -1, true>(v);
+        twiddle<R, -1>(v, tw, n2);
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) row[r2 * k1] = v[k1];
+    }
+}
+
+// z step 2 (SG = -1) and its inverse (+1, with the twiddles after): adjacent
+// threads along x.
+template <int R1, int R, int SG>
+__device__ __forceinline__ void mid_zb(c32* pl, const float2* tw, const LineGeom& g, const Team& tm) {
+    constexpr int P = R1 * R + 1;
+    const int nx = tm.x1 - tm.x0;
+    const float rX = 1.f / (float)nx;
+    for (int i = tm.t; i < nx * R1; i += tm.n) {
+        const int k1 = div_small(i, rX), x = tm.x0 + i - k1 * nx;
+        c32* row = pl + x * P + R * k1;
+        c32 v[R];
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) v[n2] = row[n2];
+        dft<R, SG, true>(v);
+        if constexpr (SG > 0) twiddle<R, 1>(v, tw, k1);
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) row[k2] = v[k2];
+    }
+}
+
+// inverse z step 1, straight to S[z][x].
+template <int R, int R2>
+__device__ __forceinline__ void mid_zo(const c32* pl, c32* S, const LineGeom& g, const Team& tm) {
+    constexpr int r2 = R2, P = R * R2 + 1;
+    const int nx = tm.x1 - tm.x0;
+    const float rX = 1.f / (float)nx;
+    for (int i = tm.t; i < nx * r2; i += tm.n) {
+        const int n2 = div_small(i, rX), x = tm.x0 + i - n2 * nx;
+        const c32* row = pl + x * P + n2;
+        c32 v[R];
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) v[k1] = row[r2 * k1];
+        dft<R, 1, true>(v);
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1)
+            if (r2 * n1 + n2 < g.Z) S[(int64_t)(r2 * n1 + n2) * g.X + x] = v[n1];
+    }
+}
+
+// depth step 1 of lines kz0 .. kz0 + nk (adjacent threads along kz).
+template <int R, int R2>
+__device__ __forceinline__ void mid_xa(const c32* pl, c32* xb, const float2* tw, const LineGeom& g,
+                                       int kz0, int nk, const Team& tm) {
+    constexpr int r2 = R2, XP = R * R2 + 1;
+    const int P = g.z.n + 1;
+    const float rn = 1.f / (float)nk;
+    for (int i = tm.t; i < nk * r2; i += tm.n) {
+        const int n2 = div_small(i, rn), kl = i - n2 * nk;
+        c32 v[R];
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) {
+            const int x = r2 * n1 + n2;
+            v[n1] = x < g.X ? pl[x * P + kz0 + kl] : 0ull;
+        }
+        dft<R, -1, true>(v);
+        twiddle<R, -1>(v, tw, n2);
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) xb[kl * XP + r2 * k1 + n2] = v[k1];
+    }
+}
+
+// depth step 2, the product with Ghat, and back.  (Ghat loaded before the barrier:
+// 0.69 against 0.55 ms for 30 volumes of 128^3, the registers spill.)
+template <int R1, int R>
+__device__ __forceinline__ void mid_xb(c32* xb, const c32* __restrict__ Gh, const float2* tw,
+                                       const LineGeom& g, int kz0, int nk, const Team& tm) {
+    constexpr int XP = R1 * R + 1;
+    const float rn = 1.f / (float)nk;
+    for (int i = tm.t; i < nk * R1; i += tm.n) {
+        const int k1 = div_small(i, rn), kl = i - k1 * nk;
+        c32 gh[R];
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) gh[k2] = __ldg(Gh + (int64_t)(R * k1 + k2) * g.z.n + kz0 + kl);
+        c32* row = xb + kl * XP + R * k1;
+        c32 v[R];
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) v[n2] = row[n2];
+        dft<R, -1, true>(v);
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) {
+            float a, b;
+            un(gh[k2], a, b);
+            v[k2] = cturn(v[k2], a, b);
+        }
+        dft<R, 1, true>(v);
+        twiddle<R, 1>(v, tw, k1);
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) row[n2] = v[n2];
+    }
+}
+
+// Frequency at a place of the transforms' order, between -N/2 and N/2.
+__device__ __forceinline__ int signed_freq(const Len& l, int pos) {
+    const int k = pos / l.r2 + l.r1 * (pos % l.r2);
+    return 2 * k > l.n ? k - l.n : k;
+}
+__device__ __forceinline__ int place_of(const Len& l, int freq) {
+    const int k = freq < 0 ? freq + l.n : freq;
+    return l.r2 * (k % l.r1) + k / l.r1;
+}
+
+// The lowest frequencies of the plane, |kz|, |ky| <= kLow, carry most of a path
+// sum (their depth correlation is nearly a running total), and a transform along
+// the depth would spread the rounding error of the largest totals evenly over the
+// depth, also to the far side where the sums are small and exp(-res) is largest.
+// They are summed directly.  Error of the attenuation maps of 61 slices of 111^2
+// against 64 bits: 1.5e-6 with none summed directly, 6.6e-7, 5.2e-7, 5.2e-7 with
+// kLow = 0, 2, 3; 5.2e-7 in the plane form, which sums all of them directly.
+constexpr int kLow = 3;
+constexpr int kLowLines = 2 * kLow + 1;
+constexpr int kLowItems = 8;     // targets per thread: 8 * kMidT >= kLowLines * X
+
+// inverse depth step 1, back into the plane (x < X).  low: the lines of the lowest
+// frequencies are left as they were.
+template <int R, int R2>
+__device__ __forceinline__ void mid_xo(c32* pl, const c32* xb, const LineGeom& g, int kz0, int nk, const Team& tm,
+                                       bool low) {
+    constexpr int r2 = R2, XP = R * R2 + 1;
+    const int P = g.z.n + 1;
+    const float rn = 1.f / (float)nk;
+    for (int i = tm.t; i < nk * r2; i += tm.n) {
+        const int n2 = div_small(i, rn), kl = i - n2 * nk;
+        c32 v[R];
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) v[k1] = xb[kl * XP + r2 * k1 + n2];
+        dft<R, 1, true>(v);
+        if (low && abs(signed_freq(g.z, kz0 + kl)) <= kLow) continue;
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) {
+            const int x = r2 * n1 + n2;
+            if (x < g.X) pl[x * P + kz0 + kl] = v[n1];
+        }
+    }
+}
+
+// Direct depth sums of the lowest kz lines, in place; G: kLowLines * D floats pairs
+// of scratch.  Scaled by Nx, as the transforms along the depth leave the others.
+__device__ __forceinline__ void mid_low(c32* pl, float2* G, const double2* __restrict__ Uf,
+                                        const double2* __restrict__ Vf, const LineGeom& g, int ky) {
+    const int P = g.z.n + 1, D = min(g.Mx, g.X);
+    for (int i = threadIdx.x; i < kLowLines * D; i += kMidT) {
+        const int j = i / D, d = i - j * D;
+        const double2 a = Uf[(int64_t)d * g.z.n + place_of(g.z, j - kLow)], b = Vf[(int64_t)d * g.y.n + ky];
+        G[i] = make_float2((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
+    }
+    __syncthreads();
+    float2 r[kLowItems];
+#pragma unroll
+    for (int q = 0; q < kLowItems; ++q) {
+        const int i = threadIdx.x + q * kMidT;
+        float2 s[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        if (i < kLowLines * g.X) {
+            const int j = i / g.X, x = i - j * g.X;
+            const c32* line = pl + x * P + place_of(g.z, j - kLow);
+            const int n = min(D, g.X - x);
+            for (int d = 0; d < n; ++d) {
+                float a, b;
+                un(line[d * P], a, b);
+                const float2 w = G[j * D + d];
+                float2& t = s[d & 1];
+                t.x = fmaf(w.x, a, fmaf(-w.y, b, t.x));
+                t.y = fmaf(w.x, b, fmaf(w.y, a, t.y));
+            }
+        }
+        const float nx = (float)g.x.n;
+        r[q] = make_float2((s[0].x + s[1].x) * nx, (s[0].y + s[1].y) * nx);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kLowItems; ++q) {
+        const int i = threadIdx.x + q * kMidT;
+        if (i < kLowLines * g.X) {
+            const int j = i / g.X, x = i - j * g.X;
+            pl[x * P + place_of(g.z, j - kLow)] = mk(r[q].x, r[q].y);
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kMidT, 1)
+line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ Gh, const double2* __restrict__ Uf,
+                const double2* __restrict__ Vf, const float2* __restrict__ Tz,
+                const float2* __restrict__ Tx, LineGeom g) {
+    extern __shared__ __align__(16) c32 sp[];
+    const int P = g.z.n + 1;
+    c32* pl = sp;                                                   // [X][Nz + 1]
+    c32* xb = pl + g.X * P;                                         // [team][G][Nx + 1]
+    float2* tz = reinterpret_cast<float2*>(xb + kMidT / g.team * g.G * (g.x.n + 1));
+    float2* tx = tz + g.z.n;
+    for (int m = threadIdx.x; m < g.z.n; m += kMidT) tz[m] = Tz[m];
+    for (int m = threadIdx.x; m < g.x.n; m += kMidT) tx[m] = Tx[m];
+    const int ky = blockIdx.x;
+    c32* Sk = S + ((int64_t)blockIdx.y * g.y.n + ky) * g.X * g.Z;
+    // the plane, eight bytes a copy, all of it in flight at once
+    const int n = g.X * g.Z;
+    const float rZ = 1.f / (float)g.Z;
+    for (int i = threadIdx.x; i < n; i += kMidT) {
+        const int x = div_small(i, rZ);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(pl + x * P + i - x * g.Z)), "l"(Sk + i));
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int teams = kMidT / g.team;
+    Team tm;
+    tm.n = g.team;
+    tm.id = threadIdx.x / g.team;
+    tm.t = threadIdx.x - tm.id * g.team;
+    tm.x0 = tm.id * g.X / teams;
+    tm.x1 = (tm.id + 1) * g.X / teams;
+    c32* xb0 = xb;
+    xb += tm.id * g.G * (g.x.n + 1);
+    const bool low = abs(signed_freq(g.y, ky)) <= kLow;
+#define CALL(A, B) mid_za<A, B>(pl, tz, g, tm)
+    FLC_LEN(g.z)
+#undef CALL
+    tm.sync();
+#define CALL(A, B) mid_zb<A, B, -1>(pl, tz, g, tm)
+    FLC_LEN(g.z)
+#undef CALL
+    __syncthreads();
+    const c32* Gk = Gh + (int64_t)ky * g.x.n * g.z.n;
+    for (int kz0 = tm.id * g.G; kz0 < g.z.n; kz0 += teams * g.G) {
+        const int nk = min(g.G, g.z.n - kz0);
+        tm.sync();
+#define CALL(A, B) mid_xa<A, B>(pl, xb, tx, g, kz0, nk, tm)
+        FLC_LEN_X(g.x)
+#undef CALL
+        tm.sync();
+#define CALL(A, B) mid_xb<A, B>(xb, Gk, tx, g, kz0, nk, tm)
+        FLC_LEN_X(g.x)
+#undef CALL
+        tm.sync();
+#define CALL(A, B) mid_xo<A, B>(pl, xb, g, kz0, nk, tm, low)
+        FLC_LEN_X(g.x)
+#undef CALL
+    }
+    __syncthreads();
+    if (low) mid_low(pl, reinterpret_cast<float2*>(xb0), Uf, Vf, g, ky);
+#define CALL(A, B) mid_zb<A, B, 1>(pl, tz, g, tm)
+    FLC_LEN(g.z)
+#undef CALL
+    tm.sync();
+#define CALL(A, B) mid_zo<A, B>(pl, Sk, g, tm)
+    FLC_LEN(g.z)
+#undef CALL
+}
+
+// ---------------------------------------------------------------------------
+// Rows inverse: grid (ceil(X / 32), Z, pairs).
+// ---------------------------------------------------------------------------
+struct OutArgs {
+    float* out;
+    int mode;                // 0 res, 1 exp(-res) in the reference layout;
+                             // 2 multiplies, 3 stores exp(-res) in the beam layout
+    int L, a_base, v0, Vn;   // first volume of this launch, volumes in all
+    int64_t a_stride, l_stride;
+    float scale;
+};
+
+template <int R1, int R>
+__device__ __forceinline__ void out_b(const c32* S, c32* sm, const float2* tw, const LineGeom& g, int nl) {
+    constexpr int P = R1 * R + 1;
+    const int64_t ks = (int64_t)g.X * g.Z;
+    const int l = threadIdx.x & 31;
+    if (l >= nl) return;
+    for (int k1 = threadIdx.x >> 5; k1 < R1; k1 += kRowsT / 32) {
+        c32 v[R];
+#pragma unroll
+        for (int k2 = 0; k2 < R; ++k2) v[k2] = S[(R * k1 + k2) * ks + l];
+        dft<R, 1, false>(v);
+        twiddle<R, 1>(v, tw, k1);
+#pragma unroll
+        for (int n2 = 0; n2 < R; ++n2) sm[l * P + R * k1 + n2] = v[n2];
+    }
+}
+
+template <int R, int R2>
+__device__ __forceinline__ void out_a(c32* sm, const LineGeom& g, const OutArgs& o, float* oa, float* ob,
+                                      int nl) {
+    constexpr int r2 = R2, P = R * R2 + 1;
+    const int l = threadIdx.x & 31;
+    if (l >= nl) return;
+    for (int n2 = threadIdx.x >> 5; n2 < r2; n2 += kRowsT / 32) {
+        c32 v[R];
+        float pa[R], pb[R];
+        if (R <= 16 && o.mode == 2) {
+            // the attenuation of these pixels, loaded before the last DFTs
+#pragma unroll
+            for (int n1 = 0; n1 < R; ++n1) {
+                const int y = r2 * n1 + n2;
+                pa[n1] = y < g.Y ? oa[(int64_t)(g.Y - 1 - y) * g.X + l] : 0.f;
+                pb[n1] = y < g.Y && ob ? ob[(int64_t)(g.Y - 1 - y) * g.X + l] : 0.f;
+            }
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < R; ++k1) v[k1] = sm[l * P + r2 * k1 + n2];
+        dft<R, 1, false>(v);
+#pragma unroll
+        for (int n1 = 0; n1 < R; ++n1) {
+            const int y = r2 * n1 + n2;
+            float ra, rb;
+            un(v[n1], ra, rb);
+            ra *= o.scale;
+            rb *= o.scale;
+            if (o.mode < 2) {
+                sm[l * P + y] = mk(o.mode ? expf(-ra) : ra, o.mode ? expf(-rb) : rb);
+            } else if (y < g.Y) {
+                const int64_t at = (int64_t)(g.Y - 1 - y) * g.X + l;
+                const float ea = expf(-ra), eb = expf(-rb);
+                oa[at] = o.mode == 2 ? (R <= 16 ? pa[n1] : oa[at]) * ea : ea;
+                if (ob) ob[at] = o.mode == 2 ? (R <= 16 ? pb[n1] : ob[at]) * eb : eb;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kRowsT, 3)
+line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArgs o, LineGeom g) {
+    extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
+    const int P = g.y.n + 1;
+    float2* tw = reinterpret_cast<float2*>(sm + kLines * P);
+    for (int m = threadIdx.x; m < g.y.n; m += kRowsT) tw[m] = Ty[m];
+    __syncthreads();
+    const int x0 = blockIdx.x * kLines, z = blockIdx.y, p = blockIdx.z;
+    const int nl = min(kLines, g.X - x0);
+    const c32* Sp = S + ((int64_t)p * g.y.n * g.Z + z) * g.X + x0;
+#define CALL(A, B) out_b<A, B>(Sp, sm, tw, g, nl)
+    FLC_LEN(g.y)
+#undef CALL
+    __syncthreads();
+    const int va = o.v0 + 2 * p, vb = va + 1;
+    float *oa, *ob;
+    if (o.mode >= 2) {
+        auto beam = [&](int v) {
+            const int al = v / o.L, l = v - al * o.L;
+            return o.out + l * o.l_stride + (int64_t)(o.a_base + al) * o.a_stride +
+                   (int64_t)z * g.Y * g.X + x0;
+        };
+        oa = beam(va);
+        ob = vb < o.Vn ? beam(vb) : nullptr;
+    } else {
+        oa = o.out + (((int64_t)va * g.Z + z) * g.X + x0) * g.Y;
+        ob = vb < o.Vn ? oa + (int64_t)g.Z * g.X * g.Y : nullptr;
+    }
+#define CALL(A, B) out_a<A, B>(sm, g, o, oa, ob, nl)
+    FLC_LEN(g.y)
+#undef CALL
+    if (o.mode >= 2) return;
+    __syncthreads();
+    const float rY = 1.f / (float)g.Y;
+    for (int i = threadIdx.x; i < nl * g.Y; i += kRowsT) {
+        const int l = div_small(i, rY), y = i - l * g.Y;
+        float ra, rb;
+        un(sm[l * P + y], ra, rb);
+        oa[i] = ra;
+        if (ob) ob[i] = rb;
+    }
+}
+
+#define FLC_ENTRY(i, A, B) {(A) * (B), A, B, i},
+const Len kLens[] = {FLC_LENS(FLC_ENTRY)};
+const Len kLensX[] = {FLC_LENS_X(FLC_ENTRY)};
+
+bool pick_len(int need, bool depth, Len* l) {
+    for (const Len& c : kLens)
+        if (c.n >= need) { *l = c; return true; }
+    if (depth)
+        for (const Len& c : kLensX)
+            if (c.n >= need) { *l = c; return true; }
+    return false;
+}
+
+size_t al256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+size_t mid_smem(const LineGeom& g) {
+    return sizeof(c32) * ((size_t)g.X * (g.z.n + 1) + (size_t)(kMidT / g.team) * g.G * (g.x.n + 1) +
+                          g.z.n + g.x.n);
+}
+size_t rows_smem(const LineGeom& g) { return sizeof(c32) * ((size_t)kLines * (g.y.n + 1) + g.y.n); }
+size_t filter_smem(const LineGeom& g) { return sizeof(c32) * ((size_t)kFilterG * (g.x.n + 1) + g.x.n); }
+
+bool line_geom(int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, LineGeom* g) {
+    if (Z < 1 || X < 1 || Y < 1 || Mz < 1 || Mx < 1 || My < 1) return false;
+    if (Z > 4096 || Y > 4096 || X > 4096 || Mx > 4096 || Mz > 4096 || My > 4096) return false;
+    const int hz = (int)Mz / 2, hy = (int)My / 2;
+    g->Z = (int)Z; g->X = (int)X; g->Y = (int)Y;
+    g->Mz = (int)Mz; g->Mx = (int)Mx; g->My = (int)My;
+    if (!pick_len((int)Z + std::max(hz, (int)Mz - 1 - hz), false, &g->z) ||
+        !pick_len((int)Y + std::max(hy, (int)My - 1 - hy), false, &g->y) ||
+        !pick_len((int)(X + std::min(Mx, X)) - 1, true, &g->x))
+        return false;
+    // teams of 256 threads, or one of all where shared memory does not hold a
+    // thread's worth of kz lines for each
+    const size_t cap = (size_t)max_smem_optin();
+    for (g->team = 256;; g->team *= 2) {
+        g->G = std::max(1, g->team / g->x.r1);
+        if (mid_smem(*g) <= cap) break;
+        if (g->team == kMidT) {
+            while (g->G > 1 && mid_smem(*g) > cap) --g->G;
+            break;
+        }
+    }
+    // (the scratch of the direct sums is a team's buffer)
+    const size_t low = sizeof(float2) * (size_t)kLowLines * std::min(g->Mx, g->X);
+    return g->G >= 4 && low <= sizeof(c32) * (size_t)(kMidT / g->team) * g->G * (g->x.n + 1) &&
+           kLowLines * g->X <= kLowItems * kMidT && kLowLines <= g->z.n && mid_smem(*g) <= cap && rows_smem(*g) <= cap && filter_smem(*g) <= cap;
+}
+
+// Pairs of volumes per pass: as many as fit in this much scratch.
+constexpr size_t kBatchBytes = 512u << 20;
+
+struct LineWs {
+    double2 *Uf, *Vf;
+    float2 *Tz, *Tx, *Ty;
+    c32 *Gh, *S;
+    int64_t batch;
+    size_t bytes;
+};
+
+LineWs line_ws(const LineGeom& g, int64_t Vn, char* base) {
+    LineWs w{};
+    size_t off = 0;
+    auto take = [&](size_t n) { char* p = base ? base + off : nullptr; off += al256(n); return p; };
+    const size_t pair = sizeof(c32) * (size_t)g.y.n * g.X * g.Z;
+    const int64_t pairs = (Vn + 1) / 2;
+    w.batch = std::max<int64_t>(1, std::min<int64_t>(pairs, (int64_t)(kBatchBytes / pair)));
+    w.batch = ceil_div(pairs, ceil_div(pairs, w.batch));            // evened
+    w.Uf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.z.n);
+    w.Vf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.y.n);
+    w.Tz = (float2*)take(sizeof(float2) * g.z.n);
+    w.Tx = (float2*)take(sizeof(float2) * g.x.n);
+    w.Ty = (float2*)take(sizeof(float2) * g.y.n);
+    w.Gh = (c32*)take(sizeof(c32) * (size_t)g.y.n * g.x.n * g.z.n);
+    w.S = (c32*)take(pair * (size_t)w.batch);
+    w.bytes = off;
+    return w;
+}
+
+template <class K>
+int allow_smem(K kernel, size_t bytes) {
+    FLC_TRY_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)bytes));
+    return FLC_OK;
+}
+
+}  // namespace
+
+// Scratch bytes of the line form for Vn volumes, 0 if it does not take the shape.
+size_t cone_line_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
+                          int64_t My) {
+    LineGeom g;
+    if (tune(kTuneConeVariant) == 5 || !line_geom(Z, X, Y, Mz, Mx, My, &g)) return 0;
+    return line_ws(g, Vn, nullptr).bytes;
+}
+
+// Scratch bytes of the spectral cone, whichever form takes the shape.
+size_t cone_spec_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
+                          int64_t My, int mode) {
+    const size_t n = cone_line_ws_bytes(Vn, Z, X, Y, Mz, Mx, My);
+    return n ? n : cone_fft_ws_bytes(Vn, Z, X, Y, Mz, Mx, My, mode);
+}
+
+// The path sum in the line form; arguments, modes and FLC_ERR_UNSUPPORTED as
+// cone_fft_launch.
+int cone_line_launch(const float* mu, const float* U, const float* Vw, float* out, int64_t Vn,
+                     int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
+                     int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, void* workspace,
+                     size_t ws_bytes, cudaStream_t st) {
+    LineGeom g;
+    if (!workspace || Vn < 1 || Vn > 65535 || tune(kTuneConeVariant) == 5 ||
+        !line_geom(Z, X, Y, Mz, Mx, My, &g) || ((uintptr_t)workspace & 255) != 0)
+        return FLC_ERR_UNSUPPORTED;
+    const LineWs w = line_ws(g, Vn, (char*)workspace);
+    if (w.bytes > ws_bytes) return FLC_ERR_UNSUPPORTED;
+    const size_t rsm = rows_smem(g), msm = mid_smem(g), fsm = filter_smem(g);
+    FLC_TRY(allow_smem(line_filter_kernel, fsm));
+    FLC_TRY(allow_smem(line_rows_kernel, rsm));
+    FLC_TRY(allow_smem(line_mid_kernel, msm));
+    FLC_TRY(allow_smem(line_out_kernel, rsm));
+    line_roots_kernel<<<(unsigned)g.Mx + 1, 256, sizeof(double2) * (size_t)(g.z.n + g.y.n), st>>>(
+        U, Vw, w.Uf, w.Vf, w.Tz, w.Tx, w.Ty, g);
+    FLC_TRY(check_launch("line_roots_kernel"));
+    line_filter_kernel<<<dim3((unsigned)g.y.n, (unsigned)ceil_div(g.z.n, kFilterG)), 256, fsm, st>>>(
+        w.Uf, w.Vf, w.Tx, w.Gh, g);
+    FLC_TRY(check_launch("line_filter_kernel"));
+    OutArgs o{out, mode, L, a_base, 0, (int)Vn, out_a_stride, out_l_stride,
+              (float)(1.0 / ((double)g.x.n * (double)g.y.n * (double)g.z.n))};
+    const int64_t vol = Z * X * Y, pairs = (Vn + 1) / 2;
+    for (int64_t p0 = 0; p0 < pairs; p0 += w.batch) {
+        const unsigned np = (unsigned)std::min<int64_t>(w.batch, pairs - p0);
+        line_rows_kernel<<<dim3((unsigned)ceil_div(Z, kLines), (unsigned)X, np), kRowsT, rsm, st>>>(
+            mu + 2 * p0 * vol, w.Ty, w.S, g, (int)(Vn - 2 * p0));
+        FLC_TRY(check_launch("line_rows_kernel"));
+        line_mid_kernel<<<dim3((unsigned)g.y.n, np), kMidT, msm, st>>>(w.S, w.Gh, w.Uf, w.Vf, w.Tz,
+                                                                       w.Tx, g);
+        FLC_TRY(check_launch("line_mid_kernel"));
+        o.v0 = (int)(2 * p0);
+        line_out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)Z, np), kRowsT, rsm, st>>>(
+            w.S, w.Ty, o, g);
+        FLC_TRY(check_launch("line_out_kernel"));
+    }
+    return FLC_OK;
+}
+
+}  // namespace flc
