@@ -927,11 +927,20 @@ size_t cone_line_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t M
     return line_ws(g, Vn, nullptr).bytes;
 }
 
+// The form tried first.  In a call over given volumes (kConeWhole), lines from four
+// on, planes below: the line form takes an odd volume at the price of two and makes a
+// larger filter (us, planes / lines: 1 volume of 64^3 85 / 98, of 128^3 151 / 189; 2 of
+// 48 x 64^2 84 / 98, of 128^3 202 / 200; 3 of 96^3 151 / 162; 4 of 20 x 150^2 194 / 164,
+// of 128^3 320 / 255).  A path that goes over its volumes in parts takes lines whatever
+// the part, so that its results don't depend on the split.
+bool cone_lines_first(int64_t Vn, int mode) { return !(mode & kConeWhole) || Vn >= 4; }
+
 // Scratch bytes of the spectral cone, whichever form takes the shape.
 size_t cone_spec_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
                           int64_t My, int mode) {
-    const size_t n = cone_line_ws_bytes(Vn, Z, X, Y, Mz, Mx, My);
-    return n ? n : cone_fft_ws_bytes(Vn, Z, X, Y, Mz, Mx, My, mode);
+    const size_t line = cone_line_ws_bytes(Vn, Z, X, Y, Mz, Mx, My);
+    const size_t plane = cone_fft_ws_bytes(Vn, Z, X, Y, Mz, Mx, My, mode & ~kConeWhole);
+    return line && (cone_lines_first(Vn, mode) || !plane) ? line : plane;
 }
 
 // The path sum in the line form; arguments, modes and FLC_ERR_UNSUPPORTED as

@@ -35,26 +35,26 @@ LENGTHS = [14, 23, 31, 38, 47, 53, 63, 70, 79, 88, 95, 107, 118, 126, 142, 159, 
 
 @pytest.mark.parametrize("n", LENGTHS)
 def test_column_lengths(n):
-    _check(2, 3, 5, n, 3, 4, 5)
+    _check(4, 3, 5, n, 3, 4, 5)
 
 
 @pytest.mark.parametrize("n", [n for n in LENGTHS if n < 330])
 def test_slice_lengths(n):
-    _check(1, n, 5, 4, 5, 3, 3)
+    _check(5, n, 5, 4, 5, 3, 3)
 
 
 @pytest.mark.parametrize("n", [n // 2 + 1 for n in LENGTHS if n < 320] + [250, 310])
 def test_depth_lengths(n):
-    _check(1, 4, n, 6, 3, n, 3)
+    _check(4, 4, n, 6, 3, n, 3)
 
 
-@pytest.mark.parametrize("K,Z,X,Y,Mz,Mx,My", [(3, 33, 35, 37, 7, 35, 9), (4, 12, 40, 9, 4, 11, 6),
-                                              (5, 7, 3, 65, 9, 12, 2), (1, 1, 1, 1, 1, 1, 1)])
+@pytest.mark.parametrize("K,Z,X,Y,Mz,Mx,My", [(7, 33, 35, 37, 7, 35, 9), (4, 12, 40, 9, 4, 11, 6),
+                                              (5, 7, 3, 65, 9, 12, 2), (4, 1, 1, 1, 1, 1, 1)])
 def test_odd_shapes(K, Z, X, Y, Mz, Mx, My):
     _check(K, Z, X, Y, Mz, Mx, My)
 
 
-@pytest.mark.parametrize("L,A,S,N", [(1, 3, 5, 34), (3, 1, 33, 20)])
+@pytest.mark.parametrize("L,A,S,N", [(1, 5, 5, 34), (3, 3, 33, 20)])
 def test_beam_layout(L, A, S, N):
     """exp(-res) multiplied into the attenuation, an odd number of volumes."""
     rng = np.random.default_rng(L + S)
