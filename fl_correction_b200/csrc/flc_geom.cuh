@@ -78,6 +78,35 @@ __device__ __forceinline__ Smp sample(const Geo& g, int h, int w) {
     return sample_xy(g, fmaf(g.c, hf, col_bx(g, w)), fmaf(g.s, hf, col_by(g, w)));
 }
 
+// Weight of position i (0 where it is 0) in a sample at x: x's fraction, or 1 less
+// it, as ffloor has it.
+__device__ __forceinline__ float tap_weight(float x, float i) {
+    return fmaxf(x >= i ? 1.f - (x - i) : x - (i - 1.f), 0.f);
+}
+
+// At an angle whose samples fall on the pixels but for the rounding of their
+// coordinates, neighbours get weights around 1e-6, and where one beam's ratio is
+// thousands of times the next one's these count.  The splats give the low row
+// v - v f, whose rounding is a few percent of such a weight (an MLEM of 14 angles of
+// 43 x 72^2 differs by 5e-4 at single pixels).  The gather kernels take the same
+// steps at these angles: part_code(x, i) is f for the high position of a sample, -f
+// (1 for f = 0) for the low one, 0 elsewhere; part_row(v, code) is the row's part and
+// part_col(part, code) the pixel's, the difference in one rounding.
+__device__ __forceinline__ bool near_axis(const Geo& g, int N) {
+    return fminf(fabsf(g.c), fabsf(g.s)) * (float)N < 0.01f;
+}
+__device__ __forceinline__ float part_code(float x, float i) {
+    const float f = x - i, h = x - (i - 1.f);
+    return f >= 1.f || h <= 0.f ? 0.f : f < 0.f ? h : f > 0.f ? -f : 1.f;
+}
+__device__ __forceinline__ float part_row(float v, float code) {
+    const float p = __fmul_rn(v, code);
+    return code < 0.f ? __fadd_rn(v, p) : p;
+}
+__device__ __forceinline__ float part_col(float v, float code) {
+    return code < 0.f ? fmaf(v, code, v) : __fmul_rn(v, code);
+}
+
 // Bilinear value of img (row stride `pitch`) at a clamped sample.
 __device__ __forceinline__ float bilerp(const float* img, int pitch, const Smp& s) {
     const float* p = img + s.i0 * pitch + s.j0;

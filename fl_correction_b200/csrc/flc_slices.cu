@@ -200,12 +200,18 @@ slices_out_kernel(const float* __restrict__ src, float* __restrict__ dst, int B,
 // ---------------------------------------------------------------------------
 constexpr int kFU = 4;     // samples whose loads are issued together
 
+// bilerp's interpolation, f = (fx, fy).
+__device__ __forceinline__ float lerp2(float2 f, float p00, float p01, float p10, float p11) {
+    const float t = fmaf(f.y, p01 - p00, p00), b = fmaf(f.y, p11 - p10, p10);
+    return fmaf(f.x, b - t, t);
+}
+
 template <int NS>
 __global__ void __launch_bounds__(kSThreads, 3)
 slices_fwd_kernel(const float* __restrict__ at, const float* __restrict__ C,
                   const float* __restrict__ em, const float* __restrict__ theta,
                   const float* __restrict__ I, float* __restrict__ out, int N, int Bp) {
-    __shared__ float4 swt[kSWarps][32];
+    __shared__ float2 swt[kSWarps][32];
     __shared__ uint32_t soff[kSWarps][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * kSWarps + warp, a = blockIdx.y;
@@ -229,9 +235,8 @@ slices_fwd_kernel(const float* __restrict__ at, const float* __restrict__ C,
         {
             const float hf = (float)(h0 + lane) - g.cy;
             const Smp s = sample_xy(g, fmaf(g.c, hf, bx), fmaf(g.s, hf, by));
-            const float gx = 1.f - s.fx, gy = 1.f - s.fy;
             __syncwarp();
-            swt[warp][lane] = make_float4(gx * gy, gx * s.fy, s.fx * gy, s.fx * s.fy);
+            swt[warp][lane] = make_float2(s.fx, s.fy);
             soff[warp][lane] = (uint32_t)(s.i0 * N + s.j0) * (uint32_t)Bp * 4u;
             __syncwarp();
         }
@@ -254,15 +259,11 @@ slices_fwd_kernel(const float* __restrict__ at, const float* __restrict__ C,
             }
 #pragma unroll
             for (int k = 0; k < kFU; ++k) {
-                const float4 q = swt[warp][k0 + k];
+                const float2 f = swt[warp][k0 + k];
 #pragma unroll
-                for (int n = 0; n < NS; ++n) {
-                    float v = q.x * v0[k][n];
-                    v = fmaf(q.y, v1[k][n], v);
-                    v = fmaf(q.z, v2[k][n], v);
-                    v = fmaf(q.w, v3[k][n], v);
-                    acc[k & 1][n] = fmaf(av[k][n], v, acc[k & 1][n]);
-                }
+                for (int n = 0; n < NS; ++n)
+                    acc[k & 1][n] =
+                        fmaf(av[k][n], lerp2(f, v0[k][n], v1[k][n], v2[k][n], v3[k][n]), acc[k & 1][n]);
             }
         }
         for (; k0 < n_h; ++k0) {
@@ -274,15 +275,10 @@ slices_fwd_kernel(const float* __restrict__ at, const float* __restrict__ C,
             load_slices<NS>(c01, o, v1);
             load_slices<NS>(c10, o, v2);
             load_slices<NS>(c11, o, v3);
-            const float4 q = swt[warp][k0];
+            const float2 f = swt[warp][k0];
 #pragma unroll
-            for (int n = 0; n < NS; ++n) {
-                float v = q.x * v0[n];
-                v = fmaf(q.y, v1[n], v);
-                v = fmaf(q.z, v2[n], v);
-                v = fmaf(q.w, v3[n], v);
-                acc[0][n] = fmaf(av[n], v, acc[0][n]);
-            }
+            for (int n = 0; n < NS; ++n)
+                acc[0][n] = fmaf(av[n], lerp2(f, v0[n], v1[n], v2[n], v3[n]), acc[0][n]);
         }
     }
     const float e = __ldg(em + a);
@@ -371,16 +367,21 @@ __device__ __forceinline__ int list_samples(const Geo& g, int N, float i, float 
         const float hf = (float)h - g.cy;
         const float x = fmaf(g.c, hf, col_bx(g, w)), y = fmaf(g.s, hf, col_by(g, w));
         const float dx = x - i, dy = y - j;
-        const float wx0 = fmaxf(1.f - fabsf(dx), 0.f), wx1 = fmaxf(1.f - fabsf(dx - 1.f), 0.f);
-        const float wy0 = fmaxf(1.f - fabsf(dy), 0.f), wy1 = fmaxf(1.f - fabsf(dy - 1.f), 0.f);
         const bool in = live && cand < 25 && (unsigned)h < (unsigned)N && (unsigned)w < (unsigned)N &&
                         x >= 0.f && x <= g.rmax && y >= 0.f && y <= g.cmax && dx > -1.f &&
                         dx < 2.f && dy > -1.f && dy < 2.f;
         const unsigned m = __ballot_sync(0xffffffffu, in) >> lead & ((1u << kSub) - 1u);
         const int at = n + __popc(m & ((1u << sub) - 1u));
         if (in && at < kSlots) {
-            const float s0 = wx0 * scale, s1 = wx1 * scale;
-            wl[at] = make_float4(s0 * wy0, s0 * wy1, s1 * wy0, s1 * wy1);
+            if (near_axis(g, N)) {
+                wl[at] = make_float4(part_code(x, i), part_code(x, i + 1.f), part_code(y, j),
+                                     part_code(y, j + 1.f));
+            } else {
+                const float s0 = fmaxf(1.f - fabsf(dx), 0.f) * scale;
+                const float s1 = fmaxf(1.f - fabsf(dx - 1.f), 0.f) * scale;
+                const float wy0 = fmaxf(1.f - fabsf(dy), 0.f), wy1 = fmaxf(1.f - fabsf(dy - 1.f), 0.f);
+                wl[at] = make_float4(s0 * wy0, s0 * wy1, s1 * wy0, s1 * wy1);
+            }
             ol[at] = make_uint2((uint32_t)(h * N + w), (uint32_t)w);
         }
         n = min(n + __popc(m), kSlots);
@@ -420,6 +421,33 @@ __device__ __forceinline__ void add_block(const float* ab, const float* rb, uint
         axpy<NS>(w.y, v[e], acc[1]);
         axpy<NS>(w.z, v[e], acc[2]);
         axpy<NS>(w.w, v[e], acc[3]);
+    }
+}
+
+// add_block at an angle near an axis: the entries are (row 0, row 1, column 0,
+// column 1) codes.
+template <int NS, bool RATIO, int E>
+__device__ __forceinline__ void add_parts(const float* ab, const float* rb, uint32_t pitch, float em,
+                                          const float4* wl, const uint2* ol, float (*acc)[NS]) {
+    float v[E][NS], r[E][NS];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint2 o = ol[e];
+        load_at<NS>(ab, o.x, pitch, v[e]);
+        if constexpr (RATIO) load_at<NS>(rb, o.y, pitch, r[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const float4 w = wl[e];
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+            const float t = __fmul_rn(v[e][n], RATIO ? __fmul_rn(r[e][n], em) : em);
+            const float t0 = part_row(t, w.x), t1 = part_row(t, w.y);
+            acc[0][n] += part_col(t0, w.z);
+            acc[1][n] += part_col(t0, w.w);
+            acc[2][n] += part_col(t1, w.z);
+            acc[3][n] += part_col(t1, w.w);
+        }
     }
 }
 
@@ -509,8 +537,7 @@ slices_frame_kernel(SArgs P) {
             const float x = fmaf(g.c, hf, col_bx(g, w)), y = fmaf(g.s, hf, col_by(g, w));
             const float o = row ? x : y;
             const float z = row ? fminf(fmaxf(y, 0.f), g.cmax) : x;
-            const float w0 = fmaxf(1.f - fabsf(z - (float)q), 0.f);
-            const float w1 = fmaxf(1.f - fabsf(z - (float)(q + 1)), 0.f);
+            const float w0 = tap_weight(z, (float)q), w1 = tap_weight(z, (float)(q + 1));
             const bool in = lane < 30 && m <= mhi && (unsigned)k < (unsigned)N &&
                             (low ? o < 0.f : o > edge) && (row || (x >= 0.f && x <= g.rmax)) &&
                             (w0 > 0.f || w1 > 0.f);
@@ -636,6 +663,17 @@ slices_bwd_kernel(SArgs P) {
         // the first eight of every block, without branches so that many loads
         // are in flight; a block that no sample reaches (outside the rotated
         // slice) has no list
+        if (near_axis(g, N)) {
+#pragma unroll
+            for (int k = 0; k < BPW; ++k) {
+                if (!(some >> k & 1u)) continue;
+#pragma unroll 1
+                for (int e = 0; e < cnts[k]; e += 2)
+                    add_parts<NS, RATIO, 2>(ab, rb, pitch, em, wl + k * L::WP + e, ol + k * L::OP + e, acc[k]);
+            }
+            if ((a - a0) % kFlush == kFlush - 1) flush();
+            continue;
+        }
         if (some == kAll) {
 #pragma unroll
             for (int k = 0; k < BPW; ++k) {
