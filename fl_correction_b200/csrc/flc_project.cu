@@ -1685,6 +1685,10 @@ bool force_band() { return use_lean() && tune(kTuneProjBand) != 0; }
 
 }  // namespace
 
+bool fwd2_takes(int64_t R, int64_t H, int64_t W) {
+    return fwd2_smem(R, H, W) <= (size_t)max_smem_optin();
+}
+
 // Lean forward (+ ratio when I != nullptr); FLC_ERR_UNSUPPORTED (nothing
 // launched) when the slice does not fit in shared memory.
 int fwd2_launch(const float* atten, const float* C, const float* em, const float* theta,
@@ -1830,9 +1834,16 @@ int bwd_emission_launch(const float* atten, const float* ratio, const float* em,
     return launch_cluster(fn, dim3(p.G, (unsigned)B), p.G, smem, st, args);
 }
 
+// Forward for few slices (flc_few.cu).
+bool use_few_fwd(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+int fwd_few_launch(const float* atten, const float* C, const float* em, const float* theta, float* out,
+                   const float* I, int64_t A, int64_t B, int64_t R, int64_t H, int64_t W,
+                   cudaStream_t st);
+
 int fwd_emission_launch(const float* atten, const float* C, const float* em, const float* theta,
                         float* Pf, const float* I, int64_t A, int64_t B, int64_t R, int64_t H,
                         int64_t W, cudaStream_t st) {
+    if (use_few_fwd(A, B, R, H, W)) return fwd_few_launch(atten, C, em, theta, Pf, I, A, B, R, H, W, st);
     if (use_lean()) {
         const int r = fwd2_launch(atten, C, em, theta, Pf, I, A, B, R, H, W, st);
         if (r != FLC_ERR_UNSUPPORTED) return r;

@@ -64,7 +64,7 @@ std::atomic<int64_t> g_tune[kTuneCount];
 const char* const kTuneNames[kTuneCount] = {"proj.cluster", "proj.apc", "cone.variant",
                                             "atten.chunk", "proj.bwd", "cone.test_wait_limit",
                                             "cone.test_skip_load", "proj.legacy", "proj.band",
-                                            "xrf.band", "proj.slices"};
+                                            "xrf.band", "proj.slices", "proj.few"};
 }  // namespace
 
 int64_t tune(int key) { return (key >= 0 && key < kTuneCount) ? g_tune[key].load() : 0; }
@@ -108,6 +108,13 @@ int mlem_iter_launch(const float* atten, const float* em, const float* theta, co
                      int64_t R, int64_t H, int64_t W, float beta, float delta, cudaStream_t st,
                      bool* fused, float* ratio_ws);
 void mlem_iter_prepare(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+
+// Gather backward for few slices (flc_few.cu); its scratch lies in MlemBufs::back.
+bool use_few(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+int bwd_few_launch(const float* atten, const float* ratio, const float* em, const float* theta,
+                   float* out, const float* Cin, const float* sens, float* frame, int64_t A, int64_t B,
+                   int64_t R, int64_t N, float clamp_min, int mode, float beta, float delta,
+                   cudaStream_t st);
 
 // MLEM on slice-fastest copies (flc_slices.cu).
 size_t mlem_slices_bytes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
@@ -170,6 +177,11 @@ size_t mlem_layout(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W, char* 
 int mlem_step(const float* atten, const float* em, const float* theta, const float* I,
               const MlemBufs& m, const float* Cin, float* Cout, int64_t A, int64_t B, int64_t R,
               int64_t H, int64_t W, float beta, float delta, cudaStream_t st) {
+    if (use_few(A, B, R, H, W)) {
+        FLC_TRY(fwd_emission_launch(atten, Cin, em, theta, m.ratio, I, A, B, R, H, W, st));
+        return bwd_few_launch(atten, m.ratio, em, theta, Cout, Cin, m.sens, m.back, A, B, R, H, 0.f, 1,
+                              beta, delta, st);
+    }
     bool fused = false;
     FLC_TRY(mlem_iter_launch(atten, em, theta, I, m.sens, Cin, Cout, A, B, R, H, W, beta, delta,
                              st, &fused, m.ratio));
@@ -249,11 +261,16 @@ extern "C" int flc_mlem(float* C, const float* atten, const float* em, const flo
     MlemBufs m;
     mlem_layout(A, B, R, H, W, (char*)workspace, &m);
     // sens = max(P^T 1, 1e-6)   (atten_cuda.cpp:308-314)
-    FLC_TRY(bwd_emission_launch(atten, nullptr, em, theta, m.sens, A, B, R, H, W, 1e-6f, st));
+    if (use_few(A, B, R, H, W))
+        FLC_TRY(bwd_few_launch(atten, nullptr, em, theta, m.sens, nullptr, nullptr, m.back, A, B, R, H, 1e-6f,
+                               0, 0.f, 0.f, st));
+    else
+        FLC_TRY(bwd_emission_launch(atten, nullptr, em, theta, m.sens, A, B, R, H, W, 1e-6f, st));
     if (n_iter == 0) return FLC_OK;
     const float fb = (float)beta, fd = (float)delta;
     const int64_t nC = R * B * H * W;
-    if (!use_graph || n_iter < 4) {
+    // (the kernels for few slices take longer than their launches: no graph to make)
+    if (!use_graph || n_iter < 4 || use_few(A, B, R, H, W)) {
         const float* cur = C;
         float* nxt = m.alt;
         for (int64_t it = 0; it < n_iter; ++it) {

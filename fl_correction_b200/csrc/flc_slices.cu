@@ -38,6 +38,14 @@ int bwd_emission_launch(const float* atten, const float* ratio, const float* em,
                         const float* theta, float* out, int64_t A, int64_t B, int64_t R,
                         int64_t H, int64_t W, float clamp_min, cudaStream_t st);
 
+// Gather backward for few slices (flc_few.cu).
+bool use_few(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W);
+int64_t few_floats(int64_t A, int64_t B, int64_t R, int64_t N);
+int bwd_few_launch(const float* atten, const float* ratio, const float* em, const float* theta,
+                   float* out, const float* Cin, const float* sens, float* frame, int64_t A, int64_t B,
+                   int64_t R, int64_t N, float clamp_min, int mode, float beta, float delta,
+                   cudaStream_t st);
+
 namespace {
 
 namespace cg = cooperative_groups;
@@ -979,7 +987,8 @@ using namespace flc;
 extern "C" size_t flc_bwd_emission_workspace_bytes(int64_t A, int64_t B, int64_t R, int64_t H,
                                                    int64_t W) {
     if (A < 1 || B < 1 || R < 1 || H < 2 || W < 2) return 0;
-    return use_slices(A, B, H, W, false) ? bwd_bytes(A, R, H, slices_pad(B)) : 0;
+    if (use_slices(A, B, H, W, false)) return bwd_bytes(A, R, H, slices_pad(B));
+    return use_few(A, B, R, H, W) ? sizeof(float) * (size_t)few_floats(A, B, R, H) : 0;
 }
 
 extern "C" int flc_bwd_emission_ws(const float* atten, const float* ratio, const float* em,
@@ -994,7 +1003,11 @@ extern "C" int flc_bwd_emission_ws(const float* atten, const float* ratio, const
         return FLC_ERR_ALIGNMENT;
     }
     const size_t need = flc_bwd_emission_workspace_bytes(A, B, R, H, W);
-    if (workspace && need && workspace_bytes >= need)
-        return bwd_slices(atten, ratio, em, theta, out, A, B, R, H, workspace, as_stream(stream));
+    if (workspace && need && workspace_bytes >= need) {
+        if (use_slices(A, B, H, W, false))
+            return bwd_slices(atten, ratio, em, theta, out, A, B, R, H, workspace, as_stream(stream));
+        return bwd_few_launch(atten, ratio, em, theta, out, nullptr, nullptr, (float*)workspace, A, B, R, H,
+                              0.f, 0, 0.f, 0.f, as_stream(stream));
+    }
     return bwd_emission_launch(atten, ratio, em, theta, out, A, B, R, H, W, 0.f, as_stream(stream));
 }

@@ -79,6 +79,9 @@ FLC_API uint64_t flc_launch_count(void);
  *   "proj.slices"   the slice-lane kernels of flc_mlem and flc_bwd_emission_ws (square
  *                   slices, where scratch is given): 1 wherever they take the shape, 2
  *                   never; automatic: from 16 slices on
+ *   "proj.few"      the gather backward for few slices of flc_mlem and
+ *                   flc_bwd_emission_ws (square slices): 1 wherever it takes the shape,
+ *                   2 never
  * Test hooks of the direct cone's bounded waits (for failure-path tests):
  *   "cone.test_wait_limit"  polls before a TMA-plane wait gives up (default 2^26)
  *   "cone.test_skip_load"   k > 0: the load of the k-th staged plane of every
