@@ -56,25 +56,20 @@ namespace {
 constexpr int kMaxCh = 8;
 constexpr int kMaxL = 8;
 
-__global__ void mul_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                           float* __restrict__ o, int64_t n) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) o[i] = a[i] * b[i];
-}
-
 __global__ void add_kernel(float* __restrict__ y, const float* __restrict__ x, int64_t n) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) y[i] += x[i];
 }
 
-// G = dL/dPf * em * bilerp(C) per sample; writes dinc = G*E (beam layout) and
-// dres = -G*atten in the depth-reversed reference layout that the cone
-// adjoint streams: dres_rev[al*L + l][s][W-1-w][H-1-h].
+// ATT = INC * E, and with G = dL/dPf * em * bilerp(C) per sample dinc = G*E (beam
+// layout) and dres = -G*ATT in the depth-reversed reference layout that the cone
+// adjoint streams: dres_rev[al*L + l][s][W-1-w][H-1-h].  (The product in this pass
+// instead of one of its own: 1.50 against 0.79 + 1.42 ms for 90 angles of 3 x 96 x 96^2.)
 // grid (ceil(W/32)*ceil(H/32), S, n_a*L), block (32, 8).
 __global__ void xrf_g_kernel(const float* __restrict__ C, const float* __restrict__ theta,
                              const float* __restrict__ em, const float* __restrict__ gPf,
-                             const float* __restrict__ ATT, const float* __restrict__ E,
-                             float* __restrict__ dinc, float* __restrict__ dres_rev, int L, int A,
+                             const float* __restrict__ INC, const float* __restrict__ E,
+                             float* __restrict__ ATT, float* __restrict__ dinc, float* __restrict__ dres_rev, int L, int A,
                              int a0, int n_a, int S, int H, int W) {
     __shared__ float T[32][33];
     const int nbw = (W + 31) >> 5;
@@ -88,17 +83,32 @@ __global__ void xrf_g_kernel(const float* __restrict__ C, const float* __restric
     const float gem = em[(int64_t)l * A + a];
     const float* gp = gPf + (((int64_t)l * A + a) * S + s) * W;
     const int64_t base = (((int64_t)l * n_a + al) * S + s) * H * W;
-    for (int k = 0; k < 32; k += 8) {
-        const int hl = threadIdx.y + k, h = h0 + hl, w = w0 + threadIdx.x;
+    const int w = w0 + threadIdx.x, h1 = h0 + threadIdx.y;
+    const float gw = w < W ? gp[w] * gem : 0.f;
+    float e[4], inc[4], c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int h = h1 + 8 * k;
+        e[k] = inc[k] = c[k] = 0.f;
+        if (h < H && w < W) {
+            const int64_t o = base + (int64_t)h * W + w;
+            e[k] = __ldg(E + o);
+            inc[k] = __ldg(INC + o);
+            c[k] = bilerp(Cl, W, sample(g, h, w));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int h = h1 + 8 * k;
         float dr = 0.f;
         if (h < H && w < W) {
-            const Smp sm = sample(g, h, w);
-            const float Gv = gp[w] * gem * bilerp(Cl, W, sm);
+            const float Gv = gw * c[k], at = inc[k] * e[k];
             const int64_t o = base + (int64_t)h * W + w;
-            dinc[o] = Gv * E[o];
-            dr = -Gv * ATT[o];
+            dinc[o] = Gv * e[k];
+            ATT[o] = at;
+            dr = -Gv * at;
         }
-        T[hl][threadIdx.x] = dr;
+        T[threadIdx.y + 8 * k][threadIdx.x] = dr;
     }
     __syncthreads();
     const int64_t vbase = (((int64_t)al * L + l) * S + s) * W;
@@ -212,10 +222,13 @@ __global__ void xrf_stage_adjoint_kernel(const float* __restrict__ frac,
 // walks the beam for line j, samples only channel j's rotated fraction and
 // writes D[j] -- the same operations in the same order as the kernel above.
 // The cone adjoint's output, stored reversed and transposed
-// ([al][l][s][W-1-w][H-1-h]), is staged through shared memory kAdjRows rows
-// at a time, so that its loads are whole sectors.  grid (L, S, n_a): the L
-// lines of one (slice, angle) are adjacent and share those rows through L2.
-// block = W rounded to 32 (up to 1024; wider slices take the kernel above).
+// ([al][l][s][W-1-w][H-1-h]), is staged through shared memory kAdjRows rows at a
+// time, a thread 32 consecutive bytes of its column and line; all lines of an (angle,
+// slice) in one block where 1024 threads hold them, so that the rows are staged once.
+// Bound by the latency of its reads: kAdjBatch rows of them in flight.  90 angles of
+// 3 x 96 x 96^2: a block per line, the staging's index divided out element by element,
+// 3.69 ms; lines together 2.35 with one row's reads at a time, 2.14 with two, 1.95
+// with four.  grid (line groups, S, n_a), block (W rounded to 32, lines).
 constexpr int kAdjRows = 8;
 
 size_t stage_adjoint_own_smem(int64_t L, int64_t W) {
@@ -223,6 +236,7 @@ size_t stage_adjoint_own_smem(int64_t L, int64_t W) {
 }
 
 constexpr int kAdjOwnMaxThreads = 1024;
+constexpr int kAdjBatch = 4;      // rows whose loads are issued together
 
 __global__ void __launch_bounds__(kAdjOwnMaxThreads)
 xrf_stage_adjoint_own_kernel(const float* __restrict__ frac, const float* __restrict__ theta,
@@ -231,13 +245,14 @@ xrf_stage_adjoint_own_kernel(const float* __restrict__ frac, const float* __rest
                              const float* __restrict__ dmu_rev, float* __restrict__ D, int n_ch,
                              int S, int H, int W, int L, int a0, int n_a) {
     extern __shared__ float sdm[];          // [L][kAdjRows][W + 1]
-    const int j = blockIdx.x, s = blockIdx.y, al = blockIdx.z, a = a0 + al, w = threadIdx.x;
-    const int P = W + 1;
-    const float cxj = __ldg(coef_x + (int64_t)a * n_ch + j);
+    const int j = blockIdx.x * blockDim.y + threadIdx.y, s = blockIdx.y, al = blockIdx.z, a = a0 + al;
+    const int w = threadIdx.x, P = W + 1;
+    const bool live = w < W && j < L;
+    const float cxj = j < L ? __ldg(coef_x + (int64_t)a * n_ch + j) : 0.f;
     float cfj[kMaxL];
 #pragma unroll
     for (int l = 0; l < kMaxL; ++l)
-        cfj[l] = l < L ? __ldg(coef_f + ((int64_t)a * L + l) * n_ch + j) : 0.f;
+        cfj[l] = l < L && j < L ? __ldg(coef_f + ((int64_t)a * L + l) * n_ch + j) : 0.f;
     const double th = (double)theta[a];
     const RotGeom g = rot_geom((float)cos(th), (float)sin(th), H, W);
     const int64_t HW = (int64_t)H * W;
@@ -249,31 +264,53 @@ xrf_stage_adjoint_own_kernel(const float* __restrict__ frac, const float* __rest
         __syncthreads();   // the previous rows have been read
         // dmu of rows h0 .. h0+nr-1: for each (line, column) nr consecutive
         // floats of the transposed layout
-        for (int t = threadIdx.x; t < L * W * nr; t += blockDim.x) {
-            const int lx = t / nr, r = t - lx * nr;
-            const int l = lx / W, x = lx - l * W;
-            sdm[(l * kAdjRows + r) * P + (W - 1 - x)] =
-                __ldg(dmu_rev + ((((int64_t)al * L + l) * S + s) * W + x) * H + (H - 1 - h0 - r));
+        for (int l = threadIdx.y; l < L; l += blockDim.y) {
+            if (w >= W) break;
+            const float* src = dmu_rev + ((((int64_t)al * L + l) * S + s) * W + w) * H + (H - 1 - h0);
+            float* dst = sdm + l * kAdjRows * P + (W - 1 - w);
+            float m[kAdjRows];
+            if (nr == kAdjRows && (H & 7) == 0) {
+                const float4 lo = __ldg(reinterpret_cast<const float4*>(src - 7));
+                const float4 hi = __ldg(reinterpret_cast<const float4*>(src - 3));
+                m[7] = lo.x; m[6] = lo.y; m[5] = lo.z; m[4] = lo.w;
+                m[3] = hi.x; m[2] = hi.y; m[1] = hi.z; m[0] = hi.w;
+            } else {
+#pragma unroll
+                for (int r = 0; r < kAdjRows; ++r) m[r] = r < nr ? __ldg(src - r) : 0.f;
+            }
+#pragma unroll
+            for (int r = 0; r < kAdjRows; ++r) dst[r * P] = m[r];
         }
         __syncthreads();
-        if (w >= W) continue;
-        // (issuing all eight rows' loads before the recursion needs 128
-        // registers and measured slower: 7.8 against 5.3 ms per 4-angle call
-        // at 256 slices of 256^2)
-        for (int r = 0; r < nr; ++r) {
-            const int h = h0 + r;
-            const RotTap tp = rot_tap(g, h, w);
-            const float fr = rot_sample_tap(fj, H, W, tp);
-            const int64_t o = o0 + (int64_t)h * W + w;
-            const float f = 1.f - fr * cxj;
-            const float di = dinc[o];
-            const float df = h > 0 ? gbar * INC[o] : 0.f;
-            gbar = h > 0 ? fmaf(gbar, f, di) : di;
-            float d = cxj * -df;
+        if (!live) continue;
+#pragma unroll 1
+        for (int q0 = 0; q0 < nr; q0 += kAdjBatch) {
+            float frq[kAdjBatch], diq[kAdjBatch], inq[kAdjBatch];
 #pragma unroll
-            for (int l = 0; l < kMaxL; ++l)
-                if (l < L) d = fmaf(cfj[l], sdm[(l * kAdjRows + r) * P + w], d);
-            D[o] = d;
+            for (int q = 0; q < kAdjBatch; ++q) {
+                const int h = min(h0 + q0 + q, H - 1);
+                const int64_t o = o0 + (int64_t)h * W + w;
+                diq[q] = __ldg(dinc + o);
+                inq[q] = __ldg(INC + o);
+            }
+#pragma unroll
+            for (int q = 0; q < kAdjBatch; ++q)
+                frq[q] = rot_sample_tap(fj, H, W, rot_tap(g, min(h0 + q0 + q, H - 1), w));
+#pragma unroll
+            for (int q = 0; q < kAdjBatch; ++q) {
+                const int r = q0 + q, h = h0 + r;
+                if (r >= nr) break;
+                const int64_t o = o0 + (int64_t)h * W + w;
+                const float f = 1.f - frq[q] * cxj;
+                const float di = diq[q];
+                const float df = h > 0 ? gbar * inq[q] : 0.f;
+                gbar = h > 0 ? fmaf(gbar, f, di) : di;
+                float d = cxj * -df;
+#pragma unroll
+                for (int l = 0; l < kMaxL; ++l)
+                    if (l < L) d = fmaf(cfj[l], sdm[(l * kAdjRows + r) * P + w], d);
+                D[o] = d;
+            }
         }
     }
 }
@@ -597,15 +634,18 @@ extern "C" int flc_xrf_project_adjoint(const float* frac, const float* theta, co
     FLC_TRY_CUDA(cudaMemsetAsync(dC, 0, sizeof(float) * L * vol, st));
     for (int64_t a0 = 0; a0 < A; a0 += chunk) {
         const int n_a = (int)(A - a0 < chunk ? A - a0 : chunk);
-        const int64_t nv = (int64_t)n_a * L * vol;
         // recompute the chunk: INC, E = exp(-cone), ATT = INC * E
         FLC_TRY(atten_stage_launch(frac, theta, coef_x, coef_f, b.INC, b.MU, (int)n_ch, (int)S,
                                    (int)H, (int)W, (int)L, vol, (int64_t)n_a * vol, (int)a0, n_a,
                                    incident_mode, 1, st, 0, x.frac4));
         FLC_TRY(cone_launch_ws(b.MU, u, v, b.E, (int64_t)n_a * L, S, W, H, Mz, Mx, My, 3, (int)L,
                                0, vol, (int64_t)n_a * vol, x.fft, x.fft_bytes, st));
-        mul_kernel<<<(unsigned)ceil_div(nv, 256), 256, 0, st>>>(b.INC, b.E, b.ATT, nv);
-        FLC_TRY(check_launch("mul_kernel"));
+        // ATT, and what goes through the attenuation
+        dim3 gg((unsigned)(ceil_div(W, 32) * ceil_div(H, 32)), (unsigned)S, (unsigned)(n_a * L));
+        xrf_g_kernel<<<gg, dim3(32, 8), 0, st>>>(frac, theta, em, gPf, b.INC, b.E, b.ATT, b.DINC,
+                                                  b.DRES, (int)L, (int)A, (int)a0, n_a, (int)S,
+                                                  (int)H, (int)W);
+        FLC_TRY(check_launch("xrf_g_kernel"));
         // direct term: P^T[atten](dL/dPf) per element
         for (int64_t l = 0; l < L; ++l) {
             FLC_TRY(bwd_emission_launch(b.ATT + l * n_a * vol, gPf + (l * A + a0) * S * W,
@@ -614,12 +654,6 @@ extern "C" int flc_xrf_project_adjoint(const float* frac, const float* theta, co
             add_kernel<<<(unsigned)ceil_div(vol, 256), 256, 0, st>>>(dC + l * vol, b.TMP, vol);
             FLC_TRY(check_launch("add_kernel"));
         }
-        // through the attenuation
-        dim3 gg((unsigned)(ceil_div(W, 32) * ceil_div(H, 32)), (unsigned)S, (unsigned)(n_a * L));
-        xrf_g_kernel<<<gg, dim3(32, 8), 0, st>>>(frac, theta, em, gPf, b.ATT, b.E, b.DINC, b.DRES,
-                                                  (int)L, (int)A, (int)a0, n_a, (int)S, (int)H,
-                                                  (int)W);
-        FLC_TRY(check_launch("xrf_g_kernel"));
         FLC_TRY(cone_launch_ws(b.DRES, uf, vf, b.DMU, (int64_t)n_a * L, S, W, H, Mz, Mx, My, 0,
                                1, 0, 0, 0, x.fft, x.fft_bytes, st));
         const int threads = (int)((W + 31) & ~31);
@@ -632,8 +666,9 @@ extern "C" int flc_xrf_project_adjoint(const float* frac, const float* theta, co
                 FLC_TRY_CUDA(cudaFuncSetAttribute(xrf_stage_adjoint_own_kernel,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)own_smem));
-            xrf_stage_adjoint_own_kernel<<<dim3((unsigned)L, (unsigned)S, (unsigned)n_a), threads,
-                                           own_smem, st>>>(
+            const int lines = (int)(threads * L <= kAdjOwnMaxThreads ? L : kAdjOwnMaxThreads / threads);
+            xrf_stage_adjoint_own_kernel<<<dim3((unsigned)ceil_div(L, lines), (unsigned)S, (unsigned)n_a),
+                                           dim3((unsigned)threads, (unsigned)lines), own_smem, st>>>(
                 frac, theta, coef_x, coef_f, b.INC, b.DINC, b.DMU, b.ATT, (int)n_ch, (int)S,
                 (int)H, (int)W, (int)L, (int)a0, n_a);
             FLC_TRY(check_launch("xrf_stage_adjoint_own_kernel"));
