@@ -74,7 +74,7 @@ struct ClusterPlan {
     size_t smem;
 };
 ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta,
-                         int threads = 512, bool uneven = false);
+                         int threads = 512);
 int launch_cluster(const void* fn, dim3 grid, int G, size_t smem, cudaStream_t st, void** args,
                    int threads = 512);
 

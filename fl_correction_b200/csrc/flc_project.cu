@@ -1486,11 +1486,8 @@ int active_clusters(const void* fn, int G, size_t smem, int threads) {
 // Cluster size G (CTAs per slice, each taking ceil(A/G) angles) minimising
 // waves * (angles per CTA + 2): the B clusters run in ceil(B / resident)
 // waves, and each CTA pays about two angles' worth of staging and reduction.
-// `uneven`: the clusters' work differs, so that they even out instead of
-// running in waves: all the work over the resident clusters, and one more
-// cluster's for the tail.  The "proj.cluster" knob forces G.
-ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta, int threads,
-                         bool uneven) {
+// The "proj.cluster" knob forces G.
+ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_cta, int threads) {
     ClusterPlan p;
     p.smem = smem_per_cta;
     int gmax = kMaxCluster < A ? kMaxCluster : (int)A;
@@ -1503,7 +1500,7 @@ ClusterPlan plan_cluster(const void* fn, int64_t A, int64_t B, size_t smem_per_c
             const int n = active_clusters(fn, G, smem_per_cta, threads);
             if (n < 1) continue;
             const int64_t item = ceil_div(A, G) + 2;
-            const int64_t cost = uneven ? B * item * 64 / n + item * 64 : ceil_div(B, n) * item;
+            const int64_t cost = ceil_div(B, n) * item;
             if (best < 0 || cost < best) {
                 best = cost;
                 best_g = G;
