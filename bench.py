@@ -90,7 +90,8 @@ def mlem_bytes_per_iter(A, S, H, W, R=1):
     return fwd + bwd + upd
 
 
-# DRAM bytes measured by ncu: the spectral cone's five kernels move 54.3 MB
+# DRAM bytes measured by ncu with the kernels that these shapes took before the
+# line-form cone and the slice-lane projector: the plane form's five kernels move 54.3 MB
 # per 128^3 volume (325.8 MB read + write for 6 volumes); an MLEM iteration
 # at the benchmark's shape (120 angles x 128 slices of 128^2, one element)
 # moves 1.026 GB in the lean forward and 1.023 GB in the lean backward,
@@ -349,29 +350,30 @@ def run_ours(args, rank, world, device):
         # the dominant kernel: the fused MLEM iteration (with the sensitivity
         # backward of each attenuation rebuild)
         "roofline": {
-            "kernel": "MLEM iteration: proj_fwd2_kernel (+ ratio) and proj_bwd2_kernel (+ update), "
+            "kernel": "MLEM iteration: slices_fwd_kernel (+ ratio), slices_frame_kernel and slices_bwd_kernel (+ update), "
                       "with the sensitivity backward of each rebuild", "bound": "hbm",
             "achieved": round(proj_gbs, 1) if proj_gbs else None, "peak": hbm, "unit": "GB/s",
             "frac": round(proj_gbs / hbm, 3) if proj_gbs else None,
             "traffic": round(MLEM_DRAM_PER_ATTEN_BYTE * 2 * A * N ** 3 * 4),
-            "traffic_note": "per element-iteration: ncu dram read + write of the lean forward and backward "
-                            "at this shape (the attenuation is read twice)",
+            "traffic_note": "per element-iteration: ncu dram read + write of the splat forward and backward "
+                            "(proj_fwd2, proj_bwd2) at this shape; the slice-lane pair reads the attenuation "
+                            "twice as well, not captured",
             "peak_kind": peak_kind,
             "algorithmic_unit": "%.4g B per element-iteration (fwd + bwd + update at the reference API "
                                 "boundary) and %.4g B per sensitivity pass (one per element and "
                                 "rebuild, %d timed)" % (bytes_it, bytes_sens, n_sens),
         },
         "roofline_cone": {
-            "kernel": "spectral cone (fft_filter, fft_fwd, fft_corr, fft_inv, fft_apply)",
+            "kernel": "spectral cone (line_roots, line_filter, line_rows, line_mid, line_out)",
             "bound": "fp32",
             "achieved": round(spec * vols_per_launch / (cone_avg_ms * 1e-3) / 1e12, 2),
             "peak": round(fp32_peak, 1),
             "unit": "TFLOP/s",
             "frac": round(spec * vols_per_launch / (cone_avg_ms * 1e-3) / 1e12 / fp32_peak, 3),
             "traffic": round(CONE_DRAM_BYTES_PER_VOLUME * vols_per_launch * (N / 128) ** 3),
-            "traffic_note": "ncu dram read+write of the five kernels on 6 volumes of 128^3, per volume, times volumes per launch",
+            "traffic_note": "ncu dram read+write of the plane form's kernels on 6 volumes of 128^3, per volume, times volumes per launch; the line form not captured",
             "peak_kind": "measured FP32 FMA rate (chain-of-FMAs probe on this pool's B200)",
-            "algorithmic_unit": "spectral FLOPs (depth correlation + 2-D FFTs, %dx%d padded planes) = %.3g per volume"
+            "algorithmic_unit": "spectral FLOPs of the plane form (direct depth correlation + 2-D FFTs, %dx%d padded planes) = %.3g per volume; the line form does fewer"
                                 % (nz_ny[0], nz_ny[1], spec),
             "launches": cone_launches, "avg_ms": round(cone_avg_ms, 4),
             "separable_equivalent_tflops": round(2 * sep * vols_per_launch / (cone_avg_ms * 1e-3) / 1e12, 1),
