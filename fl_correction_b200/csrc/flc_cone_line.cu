@@ -1,11 +1,12 @@
 // Spectral cone path sum with line transforms in registers (sm_100a).
 //
-// The algorithm is that of flc_cone_fft.cu -- the depth sum of 2-D correlations
-// as pointwise products of (z, y) spectra -- taken one axis further: along the
-// depth, R_x = sum_d G_d P_{x+d} is a correlation too, so with the depth padded
-// to Nx >= X + min(Mx, X) - 1 it is one product per frequency,
-//   Rhat(kx) = Ghat(kx) Phat(kx),  Ghat(kx) = sum_d G_d e^{+2 pi i kx d / Nx},
-// 22 instead of 66 kFLOP per frequency of a 128^3 volume.
+// The algorithm is that of flc_cone_fft.cu: the depth sum of 2-D correlations as
+// pointwise products of (z, y) spectra, R_x = sum_d G_d P_{x+d} for every frequency.
+// The depth is summed directly, as there: a transform along it (22 instead of 66 kFLOP
+// per frequency of a 128^3 volume, the middle kernel below 0.59 ms) would spread the
+// rounding error of the strongest planes, and a value that is not finite, over all of
+// them, where a plane depends on those in front of the detector only: planes 1e4 times
+// weaker in front of strong ones came out with an error of 1e-3.
 //
 // Two volumes travel together as the real and imaginary part of one complex
 // volume (the kernel is real, so the path sum acts on both alike): there are no
@@ -15,22 +16,21 @@
 // becomes X(k1 + R1 k2) at R2 k1 + k2.  The spectra stay in that order (the
 // filter is made in it), and the inverse takes the same steps back.
 //
-//   line_roots, line_filter : twiddles, the mask's line spectra, Ghat
+//   line_roots, line_filter : twiddles, the mask's line spectra, G
 //   line_rows   : mu -> S[ky][x][z]; 32 rows of one plane x per CTA, transforms
 //                 along y
 //   line_mid    : per (ky, pair of volumes), the whole (x, z) plane in shared
-//                 memory: transform along z; along x, times Ghat, back; back
+//                 memory: transform along z; the depth sums in place; back
 //                 along z; S[ky][z][x] over the same memory
 //   line_out    : transforms back along y, 32 x of one slice z per CTA, and
 //                 writes exp(-res) into the beam layout (x is its fastest axis,
 //                 so no transpose is left) or res into the reference layout
 //
-// 30 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.13, middle 0.59, out 0.23,
-// filter 0.04 ms, against 1.83 ms in five kernels of the plane form.  Rows and out
-// move the bytes they must at about half the copy rate; the middle is bound by the
-// latency of its steps (one CTA of 16 warps per SM: the plane takes 148 KB).  Teams
-// of 128 / 256 / 512 threads there: 0.60 / 0.57 / 0.66 ms; strides known at run time
-// only: 0.66; the spectra in batches small enough for L2 (40, 80 MB): 0.74, 0.71.
+// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.15, middle 1.00, out 0.20,
+// filter 0.02 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
+// the bytes they must at about half the copy rate; of the middle (one CTA of 16 warps
+// per SM: the plane takes 148 KB) 0.6 ms are the depth sums, at 58% of the FP32 rate,
+// the rest the latency of its steps.
 
 #include <algorithm>
 
@@ -207,11 +207,9 @@ __device__ __forceinline__ void dft(c32 (&v)[R]) {
         dft_pq<4, 4, SG, PK>(v);
     } else if constexpr (R == 18) {
         dft_pq<2, 9, SG, PK>(v);
-    } else if constexpr (R == 20) {
-        dft_pq<4, 5, SG, PK>(v);
     } else {
-        static_assert(R == 32, "radix");
-        dft_pq<4, 8, SG, PK>(v);
+        static_assert(R == 20, "radix");
+        dft_pq<4, 5, SG, PK>(v);
     }
 }
 
@@ -231,53 +229,45 @@ struct Len {
 
 struct LineGeom {
     int Z, X, Y, Mz, Mx, My;
-    Len z, x, y;
-    int team;       // line_mid: threads of a team,
-    int G;          // and the kz lines it takes per depth pass
+    Len z, y;
 };
 
-// Transform lengths R1 R2, as F(index, R1, R2), shortest first; the longest ones
-// for the depth only.  The steps are compiled for each, so that strides and
-// pitches are immediates.
+// Transform lengths R1 R2, as F(index, R1, R2), shortest first.  The steps
+// are compiled for each, so that strides and pitches are immediates.
 #define FLC_LENS(F)                                                                         \
     F(0, 4, 4) F(1, 6, 4) F(2, 8, 4) F(3, 8, 5) F(4, 8, 6) F(5, 9, 6) F(6, 8, 8) F(7, 9, 8) \
     F(8, 10, 8) F(9, 10, 9) F(10, 12, 8) F(11, 12, 9) F(12, 12, 10) F(13, 16, 8)            \
     F(14, 12, 12) F(15, 16, 10) F(16, 18, 10) F(17, 16, 12) F(18, 18, 12) F(19, 20, 12)     \
     F(20, 16, 16) F(21, 18, 16) F(22, 20, 16) F(23, 20, 20)
-#define FLC_LENS_X(F)                                                                       \
-    F(24, 32, 16) F(25, 32, 20)
 
 #define FLC_CASE(i, A, B) case i: CALL(A, B); break;
 #define FLC_LEN(l) switch ((l).id) { FLC_LENS(FLC_CASE) }
-#define FLC_LEN_X(l) switch ((l).id) { FLC_LENS(FLC_CASE) FLC_LENS_X(FLC_CASE) }
 
 constexpr int kRowsT = 256;      // threads of line_rows / line_out
 constexpr int kLines = 32;       // lines per CTA of line_rows / line_out
 constexpr int kMidT = 512;
+constexpr int kTeam = 256;       // threads of a team of line_mid
 
 // floor(a / b) for 0 <= a < 2^22 from b's reciprocal.
 __device__ __forceinline__ int div_small(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
 
 // ---------------------------------------------------------------------------
-// Twiddles T[m] = e^{-2 pi i m / N} of the three lengths, and the line spectra
+// Twiddles T[m] = e^{-2 pi i m / N} of the two lengths, and the line spectra
 // Uf_d(kz) = sum_dz u[d][dz] e^{+2 pi i kz (dz - hz) / Nz} (Vf likewise) in FP64,
 // in the transforms' order.  Grid Mx + 1: block d < Mx its spectra, block Mx the
 // twiddles.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 line_roots_kernel(const float* __restrict__ U, const float* __restrict__ V, double2* __restrict__ Uf,
-                  double2* __restrict__ Vf, float2* __restrict__ Tz, float2* __restrict__ Tx,
-                  float2* __restrict__ Ty, LineGeom g) {
+                  double2* __restrict__ Vf, float2* __restrict__ Tz, float2* __restrict__ Ty,
+                  LineGeom g) {
     extern __shared__ double2 root[];      // e^{2 pi i m / N} of z, then y
     const int d = blockIdx.x, Nz = g.z.n, Ny = g.y.n;
     if (d == g.Mx) {
-        for (int m = threadIdx.x; m < Nz + g.x.n + Ny; m += blockDim.x) {
-            const int n = m < Nz ? Nz : m < Nz + g.x.n ? g.x.n : Ny;
-            const int mm = m < Nz ? m : m < Nz + g.x.n ? m - Nz : m - Nz - g.x.n;
-            float2* T = m < Nz ? Tz : m < Nz + g.x.n ? Tx : Ty;
+        for (int m = threadIdx.x; m < Nz + Ny; m += blockDim.x) {
             double s, c;
-            sincospi(-2.0 * (double)mm / (double)n, &s, &c);
-            T[mm] = make_float2((float)c, (float)s);
+            sincospi(m < Nz ? -2.0 * (double)m / (double)Nz : -2.0 * (double)(m - Nz) / (double)Ny, &s, &c);
+            (m < Nz ? Tz[m] : Ty[m - Nz]) = make_float2((float)c, (float)s);
         }
         return;
     }
@@ -308,67 +298,18 @@ line_roots_kernel(const float* __restrict__ U, const float* __restrict__ V, doub
     }
 }
 
-// Ghat[ky][kx][kz] (all in the transforms' order): G_d = Uf_d(kz) Vf_d(ky), rounded
-// from FP64, transformed along d with the + sign.  Grid (Ny, ceil(Nz / 16)).
-constexpr int kFilterG = 16;
-
-template <int R, int R2>
-__device__ __forceinline__ void filter_a(const double2* Uf, const double2* Vf, c32* xb, const float2* tw,
-                                         const LineGeom& g, int ky, int kz0, int nk) {
-    constexpr int r2 = R2, P = R * R2 + 1;
-    const int D = min(g.Mx, g.X);
-    for (int i = threadIdx.x; i < kFilterG * r2; i += blockDim.x) {
-        const int kl = i % kFilterG, n2 = i / kFilterG;
-        if (kl >= nk) continue;
-        c32 v[R];
-#pragma unroll
-        for (int n1 = 0; n1 < R; ++n1) {
-            const int d = r2 * n1 + n2;
-            v[n1] = mk(0.f, 0.f);
-            if (d < D) {
-                const double2 a = Uf[(int64_t)d * g.z.n + kz0 + kl], b = Vf[(int64_t)d * g.y.n + ky];
-                v[n1] = mk((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
-            }
-        }
-        dft<R, 1, false>(v);
-        twiddle<R, 1>(v, tw, n2);
-#pragma unroll
-        for (int k1 = 0; k1 < R; ++k1) xb[kl * P + r2 * k1 + n2] = v[k1];
+// Filter spectra G[ky][d][kz] = Uf_d(kz) Vf_d(ky), d < min(Mx, X) (ky and kz in the
+// transforms' order), rounded from FP64.  Grid (D, Ny).
+__global__ void __launch_bounds__(128)
+line_filter_kernel(const double2* __restrict__ Uf, const double2* __restrict__ Vf, c32* __restrict__ G,
+                   LineGeom g) {
+    const int d = blockIdx.x, ky = blockIdx.y;
+    const double2 b = Vf[(int64_t)d * g.y.n + ky];
+    c32* Gd = G + ((int64_t)ky * gridDim.x + d) * g.z.n;
+    for (int k = threadIdx.x; k < g.z.n; k += blockDim.x) {
+        const double2 a = Uf[(int64_t)d * g.z.n + k];
+        Gd[k] = mk((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
     }
-}
-
-template <int R1, int R>
-__device__ __forceinline__ void filter_b(const c32* xb, c32* Gh, const LineGeom& g, int kz0, int nk) {
-    constexpr int P = R1 * R + 1;
-    for (int i = threadIdx.x; i < kFilterG * R1; i += blockDim.x) {
-        const int kl = i % kFilterG, k1 = i / kFilterG;
-        if (kl >= nk) continue;
-        c32 v[R];
-#pragma unroll
-        for (int n2 = 0; n2 < R; ++n2) v[n2] = xb[kl * P + R * k1 + n2];
-        dft<R, 1, false>(v);
-#pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) Gh[(int64_t)(R * k1 + k2) * g.z.n + kz0 + kl] = v[k2];
-    }
-}
-
-__global__ void __launch_bounds__(256)
-line_filter_kernel(const double2* __restrict__ Uf, const double2* __restrict__ Vf,
-                   const float2* __restrict__ Tx, c32* __restrict__ Gh, LineGeom g) {
-    extern __shared__ __align__(16) c32 sf[];
-    c32* xb = sf;                                                   // [16][Nx + 1]
-    float2* tw = reinterpret_cast<float2*>(xb + kFilterG * (g.x.n + 1));
-    for (int m = threadIdx.x; m < g.x.n; m += blockDim.x) tw[m] = Tx[m];
-    __syncthreads();
-    const int ky = blockIdx.x, kz0 = blockIdx.y * kFilterG, nk = min(kFilterG, g.z.n - kz0);
-#define CALL(A, B) filter_a<A, B>(Uf, Vf, xb, tw, g, ky, kz0, nk)
-    FLC_LEN_X(g.x)
-#undef CALL
-    __syncthreads();
-    c32* Gk = Gh + (int64_t)ky * g.x.n * g.z.n;
-#define CALL(A, B) filter_b<A, B>(xb, Gk, g, kz0, nk)
-    FLC_LEN_X(g.x)
-#undef CALL
 }
 
 // ---------------------------------------------------------------------------
@@ -438,10 +379,9 @@ line_rows_kernel(const float* __restrict__ mu, const float2* __restrict__ Ty, c3
 }
 
 // ---------------------------------------------------------------------------
-// Middle: grid (Ny, pairs), one CTA per SM with the (x, z) plane of one ky.  The
-// threads work in teams, each on its own x lines (transforms along z) and its own
-// kz lines (along the depth, in a buffer of its own), with barriers of the team
-// only: while one waits for Ghat or at a barrier, the others run.
+// Middle: grid (Ny, pairs), one CTA per SM with the (x, z) plane of one ky.  In the
+// transforms along z the threads work in teams, each on its own x lines, with barriers of
+// the team only.
 // ---------------------------------------------------------------------------
 struct Team {
     int t, n, id;     // thread in the team, threads, team
@@ -510,158 +450,86 @@ __device__ __forceinline__ void mid_zo(const c32* pl, c32* S, const LineGeom& g,
     }
 }
 
-// depth step 1 of lines kz0 .. kz0 + nk (adjacent threads along kz).
-template <int R, int R2>
-__device__ __forceinline__ void mid_xa(const c32* pl, c32* xb, const float2* tw, const LineGeom& g,
-                                       int kz0, int nk, const Team& tm) {
-    constexpr int r2 = R2, XP = R * R2 + 1;
-    const int P = g.z.n + 1;
-    const float rn = 1.f / (float)nk;
-    for (int i = tm.t; i < nk * r2; i += tm.n) {
-        const int n2 = div_small(i, rn), kl = i - n2 * nk;
-        c32 v[R];
-#pragma unroll
-        for (int n1 = 0; n1 < R; ++n1) {
-            const int x = r2 * n1 + n2;
-            v[n1] = x < g.X ? pl[x * P + kz0 + kl] : 0ull;
-        }
-        dft<R, -1, true>(v);
-        twiddle<R, -1>(v, tw, n2);
-#pragma unroll
-        for (int k1 = 0; k1 < R; ++k1) xb[kl * XP + r2 * k1 + n2] = v[k1];
-    }
-}
+// ---------------------------------------------------------------------------
+// The depth: R_x = sum_d G_d P_{x+d} for every line kz, in place.  A thread sums a tile
+// of kTile planes of one line with a window of the line in registers: per d one load
+// of the window's next plane and one of G for kTile complex products, each two paired
+// FMAs into sums of G.x P and G.y P that are put together at the end.  Tiles go in
+// rounds of a thread each, lowest planes first: a tile reads its own planes and later
+// ones, so what a round writes nobody reads any more.
+// ---------------------------------------------------------------------------
+constexpr int kTile = 12;
 
-// depth step 2, the product with Ghat, and back.  (Ghat loaded before the barrier:
-// 0.69 against 0.55 ms for 30 volumes of 128^3, the registers spill.)
-template <int R1, int R>
-__device__ __forceinline__ void mid_xb(c32* xb, const c32* __restrict__ Gh, const float2* tw,
-                                       const LineGeom& g, int kz0, int nk, const Team& tm) {
-    constexpr int XP = R1 * R + 1;
-    const float rn = 1.f / (float)nk;
-    for (int i = tm.t; i < nk * R1; i += tm.n) {
-        const int k1 = div_small(i, rn), kl = i - k1 * nk;
-        c32 gh[R];
+struct DepthSum {
+    c32 p[kTile], q[kTile], w[kTile], gv[kTile];
+    // Steps d .. d + nd - 1 of depth d's G in gv and the planes x0 + d + t in
+    // w[(d + t) % kTile]; each place is refilled for the next kTile steps as soon as it
+    // has been used (`more` of them have a G, `left` a plane).
+    template <bool FULL>
+    __device__ __forceinline__ void steps(const c32* __restrict__ G, int gs, int more, const c32* line, int P,
+                                          int left, int nd) {
 #pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) gh[k2] = __ldg(Gh + (int64_t)(R * k1 + k2) * g.z.n + kz0 + kl);
-        c32* row = xb + kl * XP + R * k1;
-        c32 v[R];
-#pragma unroll
-        for (int n2 = 0; n2 < R; ++n2) v[n2] = row[n2];
-        dft<R, -1, true>(v);
-#pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) {
+        for (int e = 0; e < kTile; ++e) {
+            if (!FULL && e >= nd) break;
             float a, b;
-            un(gh[k2], a, b);
-            v[k2] = cturn(v[k2], a, b);
-        }
-        dft<R, 1, true>(v);
-        twiddle<R, 1>(v, tw, k1);
+            un(gv[e], a, b);
+            if (FULL && e < more) gv[e] = __ldg(G + (int64_t)e * gs);
+            const c32 ga = mk(a, a), gb = mk(b, b);
 #pragma unroll
-        for (int n2 = 0; n2 < R; ++n2) row[n2] = v[n2];
-    }
-}
-
-// Frequency at a place of the transforms' order, between -N/2 and N/2.
-__device__ __forceinline__ int signed_freq(const Len& l, int pos) {
-    const int k = pos / l.r2 + l.r1 * (pos % l.r2);
-    return 2 * k > l.n ? k - l.n : k;
-}
-__device__ __forceinline__ int place_of(const Len& l, int freq) {
-    const int k = freq < 0 ? freq + l.n : freq;
-    return l.r2 * (k % l.r1) + k / l.r1;
-}
-
-// The lowest frequencies of the plane, |kz|, |ky| <= kLow, carry most of a path
-// sum (their depth correlation is nearly a running total), and a transform along
-// the depth would spread the rounding error of the largest totals evenly over the
-// depth, also to the far side where the sums are small and exp(-res) is largest.
-// They are summed directly.  Error of the attenuation maps of 61 slices of 111^2
-// against 64 bits: 1.5e-6 with none summed directly, 6.6e-7, 5.2e-7, 5.2e-7 with
-// kLow = 0, 2, 3; 5.2e-7 in the plane form, which sums all of them directly.
-constexpr int kLow = 3;
-constexpr int kLowLines = 2 * kLow + 1;
-constexpr int kLowItems = 8;     // targets per thread: 8 * kMidT >= kLowLines * X
-
-// inverse depth step 1, back into the plane (x < X).  low: the lines of the lowest
-// frequencies are left as they were.
-template <int R, int R2>
-__device__ __forceinline__ void mid_xo(c32* pl, const c32* xb, const LineGeom& g, int kz0, int nk, const Team& tm,
-                                       bool low) {
-    constexpr int r2 = R2, XP = R * R2 + 1;
-    const int P = g.z.n + 1;
-    const float rn = 1.f / (float)nk;
-    for (int i = tm.t; i < nk * r2; i += tm.n) {
-        const int n2 = div_small(i, rn), kl = i - n2 * nk;
-        c32 v[R];
-#pragma unroll
-        for (int k1 = 0; k1 < R; ++k1) v[k1] = xb[kl * XP + r2 * k1 + n2];
-        dft<R, 1, true>(v);
-        if (low && abs(signed_freq(g.z, kz0 + kl)) <= kLow) continue;
-#pragma unroll
-        for (int n1 = 0; n1 < R; ++n1) {
-            const int x = r2 * n1 + n2;
-            if (x < g.X) pl[x * P + kz0 + kl] = v[n1];
-        }
-    }
-}
-
-// Direct depth sums of the lowest kz lines, in place; G: kLowLines * D floats pairs
-// of scratch.  Scaled by Nx, as the transforms along the depth leave the others.
-__device__ __forceinline__ void mid_low(c32* pl, float2* G, const double2* __restrict__ Uf,
-                                        const double2* __restrict__ Vf, const LineGeom& g, int ky) {
-    const int P = g.z.n + 1, D = min(g.Mx, g.X);
-    for (int i = threadIdx.x; i < kLowLines * D; i += kMidT) {
-        const int j = i / D, d = i - j * D;
-        const double2 a = Uf[(int64_t)d * g.z.n + place_of(g.z, j - kLow)], b = Vf[(int64_t)d * g.y.n + ky];
-        G[i] = make_float2((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
-    }
-    __syncthreads();
-    float2 r[kLowItems];
-#pragma unroll
-    for (int q = 0; q < kLowItems; ++q) {
-        const int i = threadIdx.x + q * kMidT;
-        float2 s[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        if (i < kLowLines * g.X) {
-            const int j = i / g.X, x = i - j * g.X;
-            const c32* line = pl + x * P + place_of(g.z, j - kLow);
-            const int n = min(D, g.X - x);
-            for (int d = 0; d < n; ++d) {
-                float a, b;
-                un(line[d * P], a, b);
-                const float2 w = G[j * D + d];
-                float2& t = s[d & 1];
-                t.x = fmaf(w.x, a, fmaf(-w.y, b, t.x));
-                t.y = fmaf(w.x, b, fmaf(w.y, a, t.y));
+            for (int t = 0; t < kTile; ++t) {
+                p[t] = cfma2(ga, w[(e + t) % kTile], p[t]);
+                q[t] = cfma2(gb, w[(e + t) % kTile], q[t]);
             }
+            w[e] = e < left ? line[e * P] : 0ull;
         }
-        const float nx = (float)g.x.n;
-        r[q] = make_float2((s[0].x + s[1].x) * nx, (s[0].y + s[1].y) * nx);
     }
-    __syncthreads();
+};
+
+__device__ __forceinline__ void mid_depth(c32* pl, const c32* __restrict__ Gk, const LineGeom& g) {
+    const int Nz = g.z.n, P = Nz + 1, D = min(g.Mx, g.X);
+    const int items = Nz * ((g.X + kTile - 1) / kTile);
+    const float rN = 1.f / (float)Nz;
+    for (int i0 = 0; i0 < items; i0 += kMidT) {
+        const int i = i0 + threadIdx.x, tile = div_small(i, rN), kz = i - tile * Nz, x0 = tile * kTile;
+        const int n = i < items ? g.X - x0 : 0, dmax = min(D, n);   // planes from x0 on, depths
+        c32* line = pl + x0 * P + kz;
+        const c32* G = Gk + kz;
+        DepthSum s;
 #pragma unroll
-    for (int q = 0; q < kLowItems; ++q) {
-        const int i = threadIdx.x + q * kMidT;
-        if (i < kLowLines * g.X) {
-            const int j = i / g.X, x = i - j * g.X;
-            pl[x * P + place_of(g.z, j - kLow)] = mk(r[q].x, r[q].y);
+        for (int t = 0; t < kTile; ++t) {
+            s.p[t] = s.q[t] = 0ull;
+            s.w[t] = t < n ? line[t * P] : 0ull;
+            s.gv[t] = t < dmax ? __ldg(G + (int64_t)t * Nz) : 0ull;
+        }
+        const c32* src = line + kTile * P;
+        int left = n - kTile, d = dmax;
+#pragma unroll 1
+        for (; d >= kTile; d -= kTile) {
+            G += (int64_t)kTile * Nz;
+            s.steps<true>(G, Nz, d - kTile, src, P, left, kTile);
+            src += kTile * P;
+            left -= kTile;
+        }
+        s.steps<false>(G, Nz, 0, src, P, left, d);
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kTile; ++t) {
+            float px, py, qx, qy;
+            un(s.p[t], px, py);
+            un(s.q[t], qx, qy);
+            if (t < n) line[t * P] = mk(px - qy, py + qx);
         }
     }
     __syncthreads();
 }
 
 __global__ void __launch_bounds__(kMidT, 1)
-line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ Gh, const double2* __restrict__ Uf,
-                const double2* __restrict__ Vf, const float2* __restrict__ Tz,
-                const float2* __restrict__ Tx, LineGeom g) {
+line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ G, const float2* __restrict__ Tz, LineGeom g) {
     extern __shared__ __align__(16) c32 sp[];
     const int P = g.z.n + 1;
     c32* pl = sp;                                                   // [X][Nz + 1]
-    c32* xb = pl + g.X * P;                                         // [team][G][Nx + 1]
-    float2* tz = reinterpret_cast<float2*>(xb + kMidT / g.team * g.G * (g.x.n + 1));
-    float2* tx = tz + g.z.n;
+    float2* tz = reinterpret_cast<float2*>(pl + g.X * P);
     for (int m = threadIdx.x; m < g.z.n; m += kMidT) tz[m] = Tz[m];
-    for (int m = threadIdx.x; m < g.x.n; m += kMidT) tx[m] = Tx[m];
     const int ky = blockIdx.x;
     c32* Sk = S + ((int64_t)blockIdx.y * g.y.n + ky) * g.X * g.Z;
     // the plane, eight bytes a copy, all of it in flight at once
@@ -674,16 +542,12 @@ line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ Gh, const double2* 
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    const int teams = kMidT / g.team;
     Team tm;
-    tm.n = g.team;
-    tm.id = threadIdx.x / g.team;
-    tm.t = threadIdx.x - tm.id * g.team;
-    tm.x0 = tm.id * g.X / teams;
-    tm.x1 = (tm.id + 1) * g.X / teams;
-    c32* xb0 = xb;
-    xb += tm.id * g.G * (g.x.n + 1);
-    const bool low = abs(signed_freq(g.y, ky)) <= kLow;
+    tm.n = kTeam;
+    tm.id = threadIdx.x / kTeam;
+    tm.t = threadIdx.x - tm.id * kTeam;
+    tm.x0 = tm.id * g.X / (kMidT / kTeam);
+    tm.x1 = (tm.id + 1) * g.X / (kMidT / kTeam);
 #define CALL(A, B) mid_za<A, B>(pl, tz, g, tm)
     FLC_LEN(g.z)
 #undef CALL
@@ -692,24 +556,7 @@ line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ Gh, const double2* 
     FLC_LEN(g.z)
 #undef CALL
     __syncthreads();
-    const c32* Gk = Gh + (int64_t)ky * g.x.n * g.z.n;
-    for (int kz0 = tm.id * g.G; kz0 < g.z.n; kz0 += teams * g.G) {
-        const int nk = min(g.G, g.z.n - kz0);
-        tm.sync();
-#define CALL(A, B) mid_xa<A, B>(pl, xb, tx, g, kz0, nk, tm)
-        FLC_LEN_X(g.x)
-#undef CALL
-        tm.sync();
-#define CALL(A, B) mid_xb<A, B>(xb, Gk, tx, g, kz0, nk, tm)
-        FLC_LEN_X(g.x)
-#undef CALL
-        tm.sync();
-#define CALL(A, B) mid_xo<A, B>(pl, xb, g, kz0, nk, tm, low)
-        FLC_LEN_X(g.x)
-#undef CALL
-    }
-    __syncthreads();
-    if (low) mid_low(pl, reinterpret_cast<float2*>(xb0), Uf, Vf, g, ky);
+    mid_depth(pl, G + (int64_t)ky * min(g.Mx, g.X) * g.z.n, g);
 #define CALL(A, B) mid_zb<A, B, 1>(pl, tz, g, tm)
     FLC_LEN(g.z)
 #undef CALL
@@ -833,25 +680,17 @@ line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArg
 
 #define FLC_ENTRY(i, A, B) {(A) * (B), A, B, i},
 const Len kLens[] = {FLC_LENS(FLC_ENTRY)};
-const Len kLensX[] = {FLC_LENS_X(FLC_ENTRY)};
 
-bool pick_len(int need, bool depth, Len* l) {
+bool pick_len(int need, Len* l) {
     for (const Len& c : kLens)
         if (c.n >= need) { *l = c; return true; }
-    if (depth)
-        for (const Len& c : kLensX)
-            if (c.n >= need) { *l = c; return true; }
     return false;
 }
 
 size_t al256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-size_t mid_smem(const LineGeom& g) {
-    return sizeof(c32) * ((size_t)g.X * (g.z.n + 1) + (size_t)(kMidT / g.team) * g.G * (g.x.n + 1) +
-                          g.z.n + g.x.n);
-}
+size_t mid_smem(const LineGeom& g) { return sizeof(c32) * ((size_t)g.X * (g.z.n + 1) + g.z.n); }
 size_t rows_smem(const LineGeom& g) { return sizeof(c32) * ((size_t)kLines * (g.y.n + 1) + g.y.n); }
-size_t filter_smem(const LineGeom& g) { return sizeof(c32) * ((size_t)kFilterG * (g.x.n + 1) + g.x.n); }
 
 bool line_geom(int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, LineGeom* g) {
     if (Z < 1 || X < 1 || Y < 1 || Mz < 1 || Mx < 1 || My < 1) return false;
@@ -859,25 +698,11 @@ bool line_geom(int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t 
     const int hz = (int)Mz / 2, hy = (int)My / 2;
     g->Z = (int)Z; g->X = (int)X; g->Y = (int)Y;
     g->Mz = (int)Mz; g->Mx = (int)Mx; g->My = (int)My;
-    if (!pick_len((int)Z + std::max(hz, (int)Mz - 1 - hz), false, &g->z) ||
-        !pick_len((int)Y + std::max(hy, (int)My - 1 - hy), false, &g->y) ||
-        !pick_len((int)(X + std::min(Mx, X)) - 1, true, &g->x))
+    if (!pick_len((int)Z + std::max(hz, (int)Mz - 1 - hz), &g->z) ||
+        !pick_len((int)Y + std::max(hy, (int)My - 1 - hy), &g->y))
         return false;
-    // teams of 256 threads, or one of all where shared memory does not hold a
-    // thread's worth of kz lines for each
     const size_t cap = (size_t)max_smem_optin();
-    for (g->team = 256;; g->team *= 2) {
-        g->G = std::max(1, g->team / g->x.r1);
-        if (mid_smem(*g) <= cap) break;
-        if (g->team == kMidT) {
-            while (g->G > 1 && mid_smem(*g) > cap) --g->G;
-            break;
-        }
-    }
-    // (the scratch of the direct sums is a team's buffer)
-    const size_t low = sizeof(float2) * (size_t)kLowLines * std::min(g->Mx, g->X);
-    return g->G >= 4 && low <= sizeof(c32) * (size_t)(kMidT / g->team) * g->G * (g->x.n + 1) &&
-           kLowLines * g->X <= kLowItems * kMidT && kLowLines <= g->z.n && mid_smem(*g) <= cap && rows_smem(*g) <= cap && filter_smem(*g) <= cap;
+    return mid_smem(*g) <= cap && rows_smem(*g) <= cap;
 }
 
 // Pairs of volumes per pass: as many as fit in this much scratch.
@@ -885,8 +710,8 @@ constexpr size_t kBatchBytes = 512u << 20;
 
 struct LineWs {
     double2 *Uf, *Vf;
-    float2 *Tz, *Tx, *Ty;
-    c32 *Gh, *S;
+    float2 *Tz, *Ty;
+    c32 *G, *S;
     int64_t batch;
     size_t bytes;
 };
@@ -902,9 +727,8 @@ LineWs line_ws(const LineGeom& g, int64_t Vn, char* base) {
     w.Uf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.z.n);
     w.Vf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.y.n);
     w.Tz = (float2*)take(sizeof(float2) * g.z.n);
-    w.Tx = (float2*)take(sizeof(float2) * g.x.n);
     w.Ty = (float2*)take(sizeof(float2) * g.y.n);
-    w.Gh = (c32*)take(sizeof(c32) * (size_t)g.y.n * g.x.n * g.z.n);
+    w.G = (c32*)take(sizeof(c32) * (size_t)g.y.n * std::min(g.Mx, g.X) * g.z.n);
     w.S = (c32*)take(pair * (size_t)w.batch);
     w.bytes = off;
     return w;
@@ -955,27 +779,25 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
         return FLC_ERR_UNSUPPORTED;
     const LineWs w = line_ws(g, Vn, (char*)workspace);
     if (w.bytes > ws_bytes) return FLC_ERR_UNSUPPORTED;
-    const size_t rsm = rows_smem(g), msm = mid_smem(g), fsm = filter_smem(g);
-    FLC_TRY(allow_smem(line_filter_kernel, fsm));
+    const size_t rsm = rows_smem(g), msm = mid_smem(g);
     FLC_TRY(allow_smem(line_rows_kernel, rsm));
     FLC_TRY(allow_smem(line_mid_kernel, msm));
     FLC_TRY(allow_smem(line_out_kernel, rsm));
     line_roots_kernel<<<(unsigned)g.Mx + 1, 256, sizeof(double2) * (size_t)(g.z.n + g.y.n), st>>>(
-        U, Vw, w.Uf, w.Vf, w.Tz, w.Tx, w.Ty, g);
+        U, Vw, w.Uf, w.Vf, w.Tz, w.Ty, g);
     FLC_TRY(check_launch("line_roots_kernel"));
-    line_filter_kernel<<<dim3((unsigned)g.y.n, (unsigned)ceil_div(g.z.n, kFilterG)), 256, fsm, st>>>(
-        w.Uf, w.Vf, w.Tx, w.Gh, g);
+    line_filter_kernel<<<dim3((unsigned)std::min(g.Mx, g.X), (unsigned)g.y.n), 128, 0, st>>>(w.Uf, w.Vf, w.G,
+                                                                                             g);
     FLC_TRY(check_launch("line_filter_kernel"));
     OutArgs o{out, mode, L, a_base, 0, (int)Vn, out_a_stride, out_l_stride,
-              (float)(1.0 / ((double)g.x.n * (double)g.y.n * (double)g.z.n))};
+              (float)(1.0 / ((double)g.y.n * (double)g.z.n))};
     const int64_t vol = Z * X * Y, pairs = (Vn + 1) / 2;
     for (int64_t p0 = 0; p0 < pairs; p0 += w.batch) {
         const unsigned np = (unsigned)std::min<int64_t>(w.batch, pairs - p0);
         line_rows_kernel<<<dim3((unsigned)ceil_div(Z, kLines), (unsigned)X, np), kRowsT, rsm, st>>>(
             mu + 2 * p0 * vol, w.Ty, w.S, g, (int)(Vn - 2 * p0));
         FLC_TRY(check_launch("line_rows_kernel"));
-        line_mid_kernel<<<dim3((unsigned)g.y.n, np), kMidT, msm, st>>>(w.S, w.Gh, w.Uf, w.Vf, w.Tz,
-                                                                       w.Tx, g);
+        line_mid_kernel<<<dim3((unsigned)g.y.n, np), kMidT, msm, st>>>(w.S, w.G, w.Tz, g);
         FLC_TRY(check_launch("line_mid_kernel"));
         o.v0 = (int)(2 * p0);
         line_out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)Z, np), kRowsT, rsm, st>>>(
