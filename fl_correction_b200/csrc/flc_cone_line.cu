@@ -8,29 +8,30 @@
 // them, where a plane depends on those in front of the detector only: planes 1e4 times
 // weaker in front of strong ones came out with an error of 1e-3.
 //
-// Two volumes travel together as the real and imaginary part of one complex
-// volume (the kernel is real, so the path sum acts on both alike): there are no
-// half spectra to unpack.  Every transform has a length N = R1 R2 and runs in
-// two steps of R1- and R2-point DFTs, one line segment per thread in registers,
-// in place: element n = R2 n1 + n2 becomes A(k1, n2) at R2 k1 + n2, that
-// becomes X(k1 + R1 k2) at R2 k1 + k2.  The spectra stay in that order (the
+// Two rows of the same volume travel through the transforms along y together, as the
+// real and imaginary part of one, and are taken apart into half spectra (ky = 0 ..
+// Ny/2) before the transforms along z, so that volumes do not mix.  Every transform has
+// a length N = R1 R2 and runs in two steps of R1- and R2-point DFTs, one line segment per
+// thread in registers, in place: element n = R2 n1 + n2 becomes A(k1, n2) at R2 k1 + n2,
+// that becomes X(k1 + R1 k2) at R2 k1 + k2.  The spectra along z stay in that order (the
 // filter is made in it), and the inverse takes the same steps back.
 //
 //   line_roots, line_filter : twiddles, the mask's line spectra, G
-//   line_rows   : mu -> S[ky][x][z]; 32 rows of one plane x per CTA, transforms
+//   line_rows   : mu -> S[ky][x][z]; 64 rows of one plane x per CTA, transforms
 //                 along y
-//   line_mid    : per (ky, pair of volumes), the whole (x, z) plane in shared
-//                 memory: transform along z; the depth sums in place; back
-//                 along z; S[ky][z][x] over the same memory
-//   line_out    : transforms back along y, 32 x of one slice z per CTA, and
+//   line_mid    : per (ky, volume), the whole (x, z) plane in shared memory:
+//                 transform along z; the depth sums in place; back along z;
+//                 S[ky][z][x] over the same memory
+//   line_out    : transforms back along y, 32 x of two slices z per CTA, and
 //                 writes exp(-res) into the beam layout (x is its fastest axis,
 //                 so no transpose is left) or res into the reference layout
 //
-// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.15, middle 1.00, out 0.20,
-// filter 0.02 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
-// the bytes they must at about half the copy rate; of the middle (one CTA of 16 warps
-// per SM: the plane takes 148 KB) 0.6 ms are the depth sums, at 58% of the FP32 rate,
-// the rest the latency of its steps.
+// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.17, middle 1.00, out 0.21,
+// filter 0.01 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
+// the bytes they must at about half the copy rate (two volumes as one complex one, with
+// no half spectra to take apart: 0.15 and 0.20, but each volume then has the rounding
+// error of the other, and its NaN); of the middle (one CTA of 16 warps per SM: the plane
+// takes 148 KB) 0.77 ms are the depth sums.
 
 #include <algorithm>
 
@@ -230,6 +231,7 @@ struct Len {
 struct LineGeom {
     int Z, X, Y, Mz, Mx, My;
     Len z, y;
+    int Nyh;        // y.n / 2 + 1
 };
 
 // Transform lengths R1 R2, as F(index, R1, R2), shortest first.  The steps
@@ -244,7 +246,7 @@ struct LineGeom {
 #define FLC_LEN(l) switch ((l).id) { FLC_LENS(FLC_CASE) }
 
 constexpr int kRowsT = 256;      // threads of line_rows / line_out
-constexpr int kLines = 32;       // lines per CTA of line_rows / line_out
+constexpr int kLines = 32;       // pairs of rows per CTA of line_rows / line_out
 constexpr int kMidT = 512;
 constexpr int kTeam = 256;       // threads of a team of line_mid
 
@@ -253,7 +255,7 @@ __device__ __forceinline__ int div_small(int a, float rb) { return (int)(((float
 
 // ---------------------------------------------------------------------------
 // Twiddles T[m] = e^{-2 pi i m / N} of the two lengths, and the line spectra
-// Uf_d(kz) = sum_dz u[d][dz] e^{+2 pi i kz (dz - hz) / Nz} (Vf likewise) in FP64,
+// Uf_d(kz) = sum_dz u[d][dz] e^{+2 pi i kz (dz - hz) / Nz} (Vf likewise) in FP64, kz
 // in the transforms' order.  Grid Mx + 1: block d < Mx its spectra, block Mx the
 // twiddles.
 // ---------------------------------------------------------------------------
@@ -278,11 +280,10 @@ line_roots_kernel(const float* __restrict__ U, const float* __restrict__ V, doub
     }
     __syncthreads();
     const int hz = g.Mz / 2, hy = g.My / 2;
-    for (int p = threadIdx.x; p < Nz + Ny; p += blockDim.x) {
+    for (int p = threadIdx.x; p < Nz + g.Nyh; p += blockDim.x) {
         const bool zk = p < Nz;
-        const Len l = zk ? g.z : g.y;
-        const int pos = zk ? p : p - Nz, n = l.n, M = zk ? g.Mz : g.My, h = zk ? hz : hy;
-        const int k = pos / l.r2 + l.r1 * (pos % l.r2);      // frequency at this place
+        const int pos = zk ? p : p - Nz, n = zk ? Nz : Ny, M = zk ? g.Mz : g.My, h = zk ? hz : hy;
+        const int k = zk ? pos / g.z.r2 + g.z.r1 * (pos % g.z.r2) : pos;   // frequency at this place
         const float* w = zk ? U + (int64_t)d * g.Mz : V + (int64_t)d * g.My;
         const double2* rt = zk ? root : root + Nz;
         int m = (int)(((int64_t)k * (n - h % n)) % n);
@@ -294,17 +295,17 @@ line_roots_kernel(const float* __restrict__ U, const float* __restrict__ V, doub
             m += k;
             if (m >= n) m -= n;
         }
-        (zk ? Uf : Vf)[(int64_t)d * n + pos] = make_double2(re, im);
+        (zk ? Uf + (int64_t)d * Nz : Vf + (int64_t)d * g.Nyh)[pos] = make_double2(re, im);
     }
 }
 
-// Filter spectra G[ky][d][kz] = Uf_d(kz) Vf_d(ky), d < min(Mx, X) (ky and kz in the
-// transforms' order), rounded from FP64.  Grid (D, Ny).
+// Filter spectra G[ky][d][kz] = Uf_d(kz) Vf_d(ky), d < min(Mx, X) (kz in the transforms'
+// order), rounded from FP64.  Grid (D, Nyh).
 __global__ void __launch_bounds__(128)
 line_filter_kernel(const double2* __restrict__ Uf, const double2* __restrict__ Vf, c32* __restrict__ G,
                    LineGeom g) {
     const int d = blockIdx.x, ky = blockIdx.y;
-    const double2 b = Vf[(int64_t)d * g.y.n + ky];
+    const double2 b = Vf[(int64_t)d * g.Nyh + ky];
     c32* Gd = G + ((int64_t)ky * gridDim.x + d) * g.z.n;
     for (int k = threadIdx.x; k < g.z.n; k += blockDim.x) {
         const double2 a = Uf[(int64_t)d * g.z.n + k];
@@ -313,22 +314,28 @@ line_filter_kernel(const double2* __restrict__ Uf, const double2* __restrict__ V
 }
 
 // ---------------------------------------------------------------------------
-// Rows forward: grid (ceil(Z / 32), X, pairs).  Volume 2p is the real part,
-// 2p + 1 (if it exists) the imaginary part.
+// Rows forward: grid (ceil(Z / 64), X, volumes).  Row 2l is the real part, 2l + 1 (if
+// it exists) the imaginary part.
 // ---------------------------------------------------------------------------
+// Place of frequency k in the transforms' order.
+template <int R1, int R2>
+__device__ __forceinline__ int place(int k) { return R2 * (k % R1) + k / R1; }
+
 template <int R, int R2>
-__device__ __forceinline__ void rows_a(const float* ma, const float* mb, c32* sm, const float2* tw,
-                                       const LineGeom& g, int nl) {
+__device__ __forceinline__ void rows_a(const float* mu, c32* sm, const float2* tw, const LineGeom& g,
+                                       int nz) {
     constexpr int r2 = R2, P = R * R2 + 1;
     const int64_t zs = (int64_t)g.X * g.Y;
-    for (int i = threadIdx.x; i < nl * r2; i += kRowsT) {
+    for (int i = threadIdx.x; i < (nz + 1) / 2 * r2; i += kRowsT) {
         const int l = i / r2, n2 = i - l * r2;
+        const float* ma = mu + 2 * l * zs;
+        const bool two = 2 * l + 1 < nz;
         float a[R], b[R];
 #pragma unroll
         for (int n1 = 0; n1 < R; ++n1) {
             const int y = r2 * n1 + n2;
-            a[n1] = y < g.Y ? __ldg(ma + l * zs + y) : 0.f;
-            b[n1] = y < g.Y && mb ? __ldg(mb + l * zs + y) : 0.f;
+            a[n1] = y < g.Y ? __ldg(ma + y) : 0.f;
+            b[n1] = y < g.Y && two ? __ldg(ma + zs + y) : 0.f;
         }
         c32 v[R];
 #pragma unroll
@@ -340,46 +347,65 @@ __device__ __forceinline__ void rows_a(const float* ma, const float* mb, c32* sm
     }
 }
 
+// Step 2, then the rows' own half spectra: of the pair's W, twice the first is
+// W(k) + conj W(-k), twice the second -i (W(k) - conj W(-k)).
 template <int R1, int R>
-__device__ __forceinline__ void rows_b(const c32* sm, c32* S, const LineGeom& g, int nl) {
-    constexpr int P = R1 * R + 1;
+__device__ __forceinline__ void rows_b(c32* sm, c32* S, const LineGeom& g, int nz) {
+    constexpr int N = R1 * R, P = N + 1;
     const int64_t ks = (int64_t)g.X * g.Z;
     const int l = threadIdx.x & 31;
-    if (l >= nl) return;
-    for (int k1 = threadIdx.x >> 5; k1 < R1; k1 += kRowsT / 32) {
-        c32 v[R];
+    const bool live = 2 * l < nz;
+    if (live) {
+        for (int k1 = threadIdx.x >> 5; k1 < R1; k1 += kRowsT / 32) {
+            c32 v[R];
 #pragma unroll
-        for (int n2 = 0; n2 < R; ++n2) v[n2] = sm[l * P + R * k1 + n2];
-        dft<R, -1, false>(v);
+            for (int n2 = 0; n2 < R; ++n2) v[n2] = sm[l * P + R * k1 + n2];
+            dft<R, -1, false>(v);
 #pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) S[(R * k1 + k2) * ks + l] = v[k2];
+            for (int k2 = 0; k2 < R; ++k2) sm[l * P + R * k1 + k2] = v[k2];
+        }
+    }
+    __syncthreads();
+    if (!live) return;
+    const bool vec = (g.Z & 1) == 0;
+#pragma unroll 4
+    for (int k = threadIdx.x >> 5; k <= N / 2; k += kRowsT / 32) {
+        float x, y, u, v;
+        un(sm[l * P + place<R1, R>(k)], x, y);
+        un(sm[l * P + place<R1, R>(k ? N - k : 0)], u, v);
+        const c32 a = mk(x + u, y - v), b = mk(y + v, u - x);
+        c32* s = S + k * ks + 2 * l;
+        if (vec) {
+            *reinterpret_cast<ulonglong2*>(s) = make_ulonglong2(a, b);
+        } else {
+            s[0] = a;
+            if (2 * l + 1 < nz) s[1] = b;
+        }
     }
 }
 
 __global__ void __launch_bounds__(kRowsT, 3)
 line_rows_kernel(const float* __restrict__ mu, const float2* __restrict__ Ty, c32* __restrict__ S,
-                 LineGeom g, int Vn) {
+                 LineGeom g) {
     extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
     float2* tw = reinterpret_cast<float2*>(sm + kLines * (g.y.n + 1));
     for (int m = threadIdx.x; m < g.y.n; m += kRowsT) tw[m] = Ty[m];
     __syncthreads();
-    const int z0 = blockIdx.x * kLines, x = blockIdx.y, p = blockIdx.z;
-    const int nl = min(kLines, g.Z - z0);
-    const int64_t vol = (int64_t)g.Z * g.X * g.Y;
-    const float* ma = mu + 2 * p * vol + ((int64_t)z0 * g.X + x) * g.Y;
-    const float* mb = 2 * p + 1 < Vn ? ma + vol : nullptr;
-#define CALL(A, B) rows_a<A, B>(ma, mb, sm, tw, g, nl)
+    const int z0 = blockIdx.x * 2 * kLines, x = blockIdx.y, v = blockIdx.z;
+    const int nz = min(2 * kLines, g.Z - z0);
+    const float* src = mu + (((int64_t)v * g.Z + z0) * g.X + x) * g.Y;
+#define CALL(A, B) rows_a<A, B>(src, sm, tw, g, nz)
     FLC_LEN(g.y)
 #undef CALL
     __syncthreads();
-    c32* Sp = S + ((int64_t)p * g.y.n * g.X + x) * g.Z + z0;
-#define CALL(A, B) rows_b<A, B>(sm, Sp, g, nl)
+    c32* Sv = S + ((int64_t)v * g.Nyh * g.X + x) * g.Z + z0;
+#define CALL(A, B) rows_b<A, B>(sm, Sv, g, nz)
     FLC_LEN(g.y)
 #undef CALL
 }
 
 // ---------------------------------------------------------------------------
-// Middle: grid (Ny, pairs), one CTA per SM with the (x, z) plane of one ky.  In the
+// Middle: grid (Nyh, volumes), one CTA per SM with the (x, z) plane of one ky.  In the
 // transforms along z the threads work in teams, each on its own x lines, with barriers of
 // the team only.
 // ---------------------------------------------------------------------------
@@ -531,7 +557,7 @@ line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ G, const float2* __
     float2* tz = reinterpret_cast<float2*>(pl + g.X * P);
     for (int m = threadIdx.x; m < g.z.n; m += kMidT) tz[m] = Tz[m];
     const int ky = blockIdx.x;
-    c32* Sk = S + ((int64_t)blockIdx.y * g.y.n + ky) * g.X * g.Z;
+    c32* Sk = S + ((int64_t)blockIdx.y * g.Nyh + ky) * g.X * g.Z;
     // the plane, eight bytes a copy, all of it in flight at once
     const int n = g.X * g.Z;
     const float rZ = 1.f / (float)g.Z;
@@ -567,27 +593,42 @@ line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ G, const float2* __
 }
 
 // ---------------------------------------------------------------------------
-// Rows inverse: grid (ceil(X / 32), Z, pairs).
+// Rows inverse: grid (ceil(X / 32), ceil(Z / 2), volumes).  Slices z and z + 1 (if it
+// exists) are the real and the imaginary part.
 // ---------------------------------------------------------------------------
 struct OutArgs {
     float* out;
     int mode;                // 0 res, 1 exp(-res) in the reference layout;
                              // 2 multiplies, 3 stores exp(-res) in the beam layout
-    int L, a_base, v0, Vn;   // first volume of this launch, volumes in all
+    int L, a_base, v0;       // first volume of this launch
     int64_t a_stride, l_stride;
     float scale;
 };
 
+// The slices' half spectra as one spectrum, then step 1.
 template <int R1, int R>
-__device__ __forceinline__ void out_b(const c32* S, c32* sm, const float2* tw, const LineGeom& g, int nl) {
-    constexpr int P = R1 * R + 1;
+__device__ __forceinline__ void out_b(const c32* S, c32* sm, const float2* tw, const LineGeom& g, int nl,
+                                      bool two) {
+    constexpr int N = R1 * R, P = N + 1;
     const int64_t ks = (int64_t)g.X * g.Z;
     const int l = threadIdx.x & 31;
+    if (l < nl) {
+#pragma unroll 4
+        for (int k = threadIdx.x >> 5; k <= N / 2; k += kRowsT / 32) {
+            float x, y, u = 0.f, v = 0.f;
+            un(S[k * ks + l], x, y);
+            if (two) un(S[k * ks + g.X + l], u, v);
+            if (k == 0 || 2 * k == N) y = v = 0.f;       // (real rows)
+            sm[l * P + place<R1, R>(k)] = mk(x - v, y + u);
+            if (k != 0 && 2 * k != N) sm[l * P + place<R1, R>(N - k)] = mk(x + v, u - y);
+        }
+    }
+    __syncthreads();
     if (l >= nl) return;
     for (int k1 = threadIdx.x >> 5; k1 < R1; k1 += kRowsT / 32) {
         c32 v[R];
 #pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) v[k2] = S[(R * k1 + k2) * ks + l];
+        for (int k2 = 0; k2 < R; ++k2) v[k2] = sm[l * P + R * k1 + k2];
         dft<R, 1, false>(v);
         twiddle<R, 1>(v, tw, k1);
 #pragma unroll
@@ -642,27 +683,23 @@ line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArg
     float2* tw = reinterpret_cast<float2*>(sm + kLines * P);
     for (int m = threadIdx.x; m < g.y.n; m += kRowsT) tw[m] = Ty[m];
     __syncthreads();
-    const int x0 = blockIdx.x * kLines, z = blockIdx.y, p = blockIdx.z;
+    const int x0 = blockIdx.x * kLines, z = 2 * blockIdx.y;
+    const bool two = z + 1 < g.Z;
     const int nl = min(kLines, g.X - x0);
-    const c32* Sp = S + ((int64_t)p * g.y.n * g.Z + z) * g.X + x0;
-#define CALL(A, B) out_b<A, B>(Sp, sm, tw, g, nl)
+    const c32* Sv = S + ((int64_t)blockIdx.z * g.Nyh * g.Z + z) * g.X + x0;
+#define CALL(A, B) out_b<A, B>(Sv, sm, tw, g, nl, two)
     FLC_LEN(g.y)
 #undef CALL
     __syncthreads();
-    const int va = o.v0 + 2 * p, vb = va + 1;
-    float *oa, *ob;
+    const int v = o.v0 + blockIdx.z;
+    float* oa;
     if (o.mode >= 2) {
-        auto beam = [&](int v) {
-            const int al = v / o.L, l = v - al * o.L;
-            return o.out + l * o.l_stride + (int64_t)(o.a_base + al) * o.a_stride +
-                   (int64_t)z * g.Y * g.X + x0;
-        };
-        oa = beam(va);
-        ob = vb < o.Vn ? beam(vb) : nullptr;
+        const int al = v / o.L, l = v - al * o.L;
+        oa = o.out + l * o.l_stride + (int64_t)(o.a_base + al) * o.a_stride + (int64_t)z * g.Y * g.X + x0;
     } else {
-        oa = o.out + (((int64_t)va * g.Z + z) * g.X + x0) * g.Y;
-        ob = vb < o.Vn ? oa + (int64_t)g.Z * g.X * g.Y : nullptr;
+        oa = o.out + (((int64_t)v * g.Z + z) * g.X + x0) * g.Y;
     }
+    float* ob = two ? oa + (int64_t)g.X * g.Y : nullptr;
 #define CALL(A, B) out_a<A, B>(sm, g, o, oa, ob, nl)
     FLC_LEN(g.y)
 #undef CALL
@@ -701,11 +738,12 @@ bool line_geom(int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t 
     if (!pick_len((int)Z + std::max(hz, (int)Mz - 1 - hz), &g->z) ||
         !pick_len((int)Y + std::max(hy, (int)My - 1 - hy), &g->y))
         return false;
+    g->Nyh = g->y.n / 2 + 1;
     const size_t cap = (size_t)max_smem_optin();
     return mid_smem(*g) <= cap && rows_smem(*g) <= cap;
 }
 
-// Pairs of volumes per pass: as many as fit in this much scratch.
+// Volumes per pass: as many as fit in this much scratch.
 constexpr size_t kBatchBytes = 512u << 20;
 
 struct LineWs {
@@ -720,16 +758,15 @@ LineWs line_ws(const LineGeom& g, int64_t Vn, char* base) {
     LineWs w{};
     size_t off = 0;
     auto take = [&](size_t n) { char* p = base ? base + off : nullptr; off += al256(n); return p; };
-    const size_t pair = sizeof(c32) * (size_t)g.y.n * g.X * g.Z;
-    const int64_t pairs = (Vn + 1) / 2;
-    w.batch = std::max<int64_t>(1, std::min<int64_t>(pairs, (int64_t)(kBatchBytes / pair)));
-    w.batch = ceil_div(pairs, ceil_div(pairs, w.batch));            // evened
+    const size_t vol = sizeof(c32) * (size_t)g.Nyh * g.X * g.Z;
+    w.batch = std::max<int64_t>(1, std::min<int64_t>(Vn, (int64_t)(kBatchBytes / vol)));
+    w.batch = ceil_div(Vn, ceil_div(Vn, w.batch));                  // evened
     w.Uf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.z.n);
-    w.Vf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.y.n);
+    w.Vf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.Nyh);
     w.Tz = (float2*)take(sizeof(float2) * g.z.n);
     w.Ty = (float2*)take(sizeof(float2) * g.y.n);
-    w.G = (c32*)take(sizeof(c32) * (size_t)g.y.n * std::min(g.Mx, g.X) * g.z.n);
-    w.S = (c32*)take(pair * (size_t)w.batch);
+    w.G = (c32*)take(sizeof(c32) * (size_t)g.Nyh * std::min(g.Mx, g.X) * g.z.n);
+    w.S = (c32*)take(vol * (size_t)w.batch);
     w.bytes = off;
     return w;
 }
@@ -752,8 +789,7 @@ size_t cone_line_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t M
 }
 
 // The form tried first.  In a call over given volumes (kConeWhole), lines from four
-// on, planes below: the line form takes an odd volume at the price of two and makes a
-// larger filter (us, planes / lines: 1 volume of 64^3 85 / 98, of 128^3 151 / 189; 2 of
+// on, planes below (us, planes / lines: 1 volume of 64^3 85 / 98, of 128^3 151 / 189; 2 of
 // 48 x 64^2 84 / 98, of 128^3 202 / 200; 3 of 96^3 151 / 162; 4 of 20 x 150^2 194 / 164,
 // of 128^3 320 / 255).  A path that goes over its volumes in parts takes lines whatever
 // the part, so that its results don't depend on the split.
@@ -786,21 +822,21 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
     line_roots_kernel<<<(unsigned)g.Mx + 1, 256, sizeof(double2) * (size_t)(g.z.n + g.y.n), st>>>(
         U, Vw, w.Uf, w.Vf, w.Tz, w.Ty, g);
     FLC_TRY(check_launch("line_roots_kernel"));
-    line_filter_kernel<<<dim3((unsigned)std::min(g.Mx, g.X), (unsigned)g.y.n), 128, 0, st>>>(w.Uf, w.Vf, w.G,
+    line_filter_kernel<<<dim3((unsigned)std::min(g.Mx, g.X), (unsigned)g.Nyh), 128, 0, st>>>(w.Uf, w.Vf, w.G,
                                                                                              g);
     FLC_TRY(check_launch("line_filter_kernel"));
-    OutArgs o{out, mode, L, a_base, 0, (int)Vn, out_a_stride, out_l_stride,
-              (float)(1.0 / ((double)g.y.n * (double)g.z.n))};
-    const int64_t vol = Z * X * Y, pairs = (Vn + 1) / 2;
-    for (int64_t p0 = 0; p0 < pairs; p0 += w.batch) {
-        const unsigned np = (unsigned)std::min<int64_t>(w.batch, pairs - p0);
-        line_rows_kernel<<<dim3((unsigned)ceil_div(Z, kLines), (unsigned)X, np), kRowsT, rsm, st>>>(
-            mu + 2 * p0 * vol, w.Ty, w.S, g, (int)(Vn - 2 * p0));
+    OutArgs o{out, mode, L, a_base, 0, out_a_stride, out_l_stride,
+              (float)(0.5 / ((double)g.y.n * (double)g.z.n))};      // (line_rows leaves twice the spectra)
+    const int64_t vol = Z * X * Y;
+    for (int64_t v0 = 0; v0 < Vn; v0 += w.batch) {
+        const unsigned n = (unsigned)std::min<int64_t>(w.batch, Vn - v0);
+        line_rows_kernel<<<dim3((unsigned)ceil_div(Z, 2 * kLines), (unsigned)X, n), kRowsT, rsm, st>>>(
+            mu + v0 * vol, w.Ty, w.S, g);
         FLC_TRY(check_launch("line_rows_kernel"));
-        line_mid_kernel<<<dim3((unsigned)g.y.n, np), kMidT, msm, st>>>(w.S, w.G, w.Tz, g);
+        line_mid_kernel<<<dim3((unsigned)g.Nyh, n), kMidT, msm, st>>>(w.S, w.G, w.Tz, g);
         FLC_TRY(check_launch("line_mid_kernel"));
-        o.v0 = (int)(2 * p0);
-        line_out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)Z, np), kRowsT, rsm, st>>>(
+        o.v0 = (int)v0;
+        line_out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)ceil_div(Z, 2), n), kRowsT, rsm, st>>>(
             w.S, w.Ty, o, g);
         FLC_TRY(check_launch("line_out_kernel"));
     }

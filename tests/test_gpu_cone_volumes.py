@@ -6,8 +6,10 @@ import pytest
 import torch
 
 from fl_correction_b200.cuda_lib import cal_atten_cuda
+from fl_correction_b200.xrf import XRFProjector
 from helpers import TOL_MAP, T
 from oracle import oracle as O
+from test_gpu_xrf import _case as _xrf_case
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +49,35 @@ def test_non_finite_plane_stays_behind(bad):
         out = cal_atten_cuda(T(mu[:K]), T(mask)).cpu().numpy()
         assert not np.isfinite(out[0, 3, x, 5])
         assert _plane_err(out[:1, :, x + 1:], ref[:1, :, x + 1:]).max() < TOL_MAP
+
+
+SCALES = np.array([1.0, 1e-4, 1e3, 1e-2, 1.0], np.float32)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_volumes_of_unequal_scale(shape):
+    mu, mask = _case(*shape)
+    mu *= SCALES[:shape[0], None, None, None]
+    out = cal_atten_cuda(T(mu), T(mask)).cpu().numpy()
+    assert _plane_err(out, O.cone_ref(mu, mask)).max() < TOL_MAP
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_volumes_do_not_see_each_other(shape):
+    """A volume's bits, whatever the others hold."""
+    mu, mask = _case(*shape)
+    out = cal_atten_cuda(T(mu), T(mask))
+    for v in range(shape[0]):
+        other = np.full_like(mu, np.nan)
+        other[v] = mu[v]
+        assert torch.equal(cal_atten_cuda(T(other), T(mask))[v], out[v])
+
+
+@pytest.mark.parametrize("chunk", [1, 3, 4])
+def test_lines_in_odd_chunks(chunk):
+    """Three lines over parts of the angles: the same bits as over all of them."""
+    p, angles, mask, frac, rng = _xrf_case(21, n_ch=3, L=3, S=5, N=24, A=7)
+    S, N = frac.shape[1], frac.shape[-1]
+    full = XRFProjector(p, angles, mask, (S, N, N))
+    part = XRFProjector(p, angles, mask, (S, N, N), chunk=chunk)
+    assert torch.equal(full.project(T(frac)), part.project(T(frac)))
