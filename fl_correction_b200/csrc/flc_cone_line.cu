@@ -26,12 +26,12 @@
 //                 writes exp(-res) into the beam layout (x is its fastest axis,
 //                 so no transpose is left) or res into the reference layout
 //
-// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.17, middle 1.00, out 0.21,
+// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.17, middle 0.85, out 0.21,
 // filter 0.01 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
 // the bytes they must at about half the copy rate (two volumes as one complex one, with
 // no half spectra to take apart: 0.15 and 0.20, but each volume then has the rounding
 // error of the other, and its NaN); of the middle (one CTA of 16 warps per SM: the plane
-// takes 148 KB) 0.77 ms are the depth sums.
+// takes 148 KB) 0.6 ms are the depth sums.
 
 #include <algorithm>
 
@@ -480,17 +480,23 @@ __device__ __forceinline__ void mid_zo(const c32* pl, c32* S, const LineGeom& g,
 // The depth: R_x = sum_d G_d P_{x+d} for every line kz, in place.  A thread sums a tile
 // of kTile planes of one line with a window of the line in registers: per d one load
 // of the window's next plane and one of G for kTile complex products, each two paired
-// FMAs into sums of G.x P and G.y P that are put together at the end.  Tiles go in
+// FMAs into sums of G.x P and G.y P that are put together every kRun depths.  Tiles go in
 // rounds of a thread each, lowest planes first: a tile reads its own planes and later
-// ones, so what a round writes nobody reads any more.
+// ones, so what a round writes nobody reads any more.  Middle kernel, 36 volumes of 128^3:
+// tiles of 12 planes 1.00 ms, 10 0.94, 8 0.82, 6 0.89 (four warps a scheduler, and what
+// the registers leave for loads in flight; 768 threads of 80 registers 1.06); the sums cut
+// at 64 depths and G four steps ahead instead of eight 0.85, eight steps ahead 0.92, the
+// depths in halves on two lanes 0.94.
 // ---------------------------------------------------------------------------
-constexpr int kTile = 12;
+constexpr int kTile = 8;
+constexpr int kAhead = 4;        // steps that G is loaded ahead of its use
+constexpr int kRun = 64;         // depths summed in one go: short sums, for their rounding error
 
 struct DepthSum {
-    c32 p[kTile], q[kTile], w[kTile], gv[kTile];
-    // Steps d .. d + nd - 1 of depth d's G in gv and the planes x0 + d + t in
-    // w[(d + t) % kTile]; each place is refilled for the next kTile steps as soon as it
-    // has been used (`more` of them have a G, `left` a plane).
+    c32 p[kTile], q[kTile], w[kTile], gv[kAhead], sum[kTile];
+    // Steps d .. d + nd - 1, the planes x0 + d + t in w[(d + t) % kTile]; each place of
+    // w and gv is refilled as soon as it has been used (`more` depths from `G` on exist,
+    // `left` planes from `line` on).
     template <bool FULL>
     __device__ __forceinline__ void steps(const c32* __restrict__ G, int gs, int more, const c32* line, int P,
                                           int left, int nd) {
@@ -498,8 +504,8 @@ struct DepthSum {
         for (int e = 0; e < kTile; ++e) {
             if (!FULL && e >= nd) break;
             float a, b;
-            un(gv[e], a, b);
-            if (FULL && e < more) gv[e] = __ldg(G + (int64_t)e * gs);
+            un(gv[e % kAhead], a, b);
+            if (e < more) gv[e % kAhead] = __ldg(G + (int64_t)e * gs);
             const c32 ga = mk(a, a), gb = mk(b, b);
 #pragma unroll
             for (int t = 0; t < kTile; ++t) {
@@ -507,6 +513,16 @@ struct DepthSum {
                 q[t] = cfma2(gb, w[(e + t) % kTile], q[t]);
             }
             w[e] = e < left ? line[e * P] : 0ull;
+        }
+    }
+    __device__ __forceinline__ void flush() {
+#pragma unroll
+        for (int t = 0; t < kTile; ++t) {
+            float px, py, qx, qy;
+            un(p[t], px, py);
+            un(q[t], qx, qy);
+            sum[t] = cadd<true>(sum[t], mk(px - qy, py + qx));
+            p[t] = q[t] = 0ull;
         }
     }
 };
@@ -523,28 +539,27 @@ __device__ __forceinline__ void mid_depth(c32* pl, const c32* __restrict__ Gk, c
         DepthSum s;
 #pragma unroll
         for (int t = 0; t < kTile; ++t) {
-            s.p[t] = s.q[t] = 0ull;
+            s.p[t] = s.q[t] = s.sum[t] = 0ull;
             s.w[t] = t < n ? line[t * P] : 0ull;
-            s.gv[t] = t < dmax ? __ldg(G + (int64_t)t * Nz) : 0ull;
+            if (t < kAhead) s.gv[t] = t < dmax ? __ldg(G + (int64_t)t * Nz) : 0ull;
         }
         const c32* src = line + kTile * P;
+        G += (int64_t)kAhead * Nz;
         int left = n - kTile, d = dmax;
 #pragma unroll 1
         for (; d >= kTile; d -= kTile) {
+            s.steps<true>(G, Nz, d - kAhead, src, P, left, kTile);
             G += (int64_t)kTile * Nz;
-            s.steps<true>(G, Nz, d - kTile, src, P, left, kTile);
             src += kTile * P;
             left -= kTile;
+            if ((dmax - d) % kRun == kRun - kTile) s.flush();
         }
-        s.steps<false>(G, Nz, 0, src, P, left, d);
+        s.steps<false>(G, Nz, d - kAhead, src, P, left, d);
+        s.flush();
         __syncthreads();
 #pragma unroll
-        for (int t = 0; t < kTile; ++t) {
-            float px, py, qx, qy;
-            un(s.p[t], px, py);
-            un(s.q[t], qx, qy);
-            if (t < n) line[t * P] = mk(px - qy, py + qx);
-        }
+        for (int t = 0; t < kTile; ++t)
+            if (t < n) line[t * P] = s.sum[t];
     }
     __syncthreads();
 }
