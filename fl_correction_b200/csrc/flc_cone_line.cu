@@ -26,11 +26,11 @@
 //                 writes exp(-res) into the beam layout (x is its fastest axis,
 //                 so no transpose is left) or res into the reference layout
 //
-// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.17, middle 0.85, out 0.21,
+// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.16, middle 0.87, out 0.18,
 // filter 0.01 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
-// the bytes they must at about half the copy rate (two volumes as one complex one, with
-// no half spectra to take apart: 0.15 and 0.20, but each volume then has the rounding
-// error of the other, and its NaN); of the middle (one CTA of 16 warps per SM: the plane
+// the bytes they must at about half the copy rate, four CTAs an SM (three: 0.17 and 0.21;
+// two volumes as one complex one, with no half spectra to take apart, three CTAs: 0.15
+// and 0.20, but each volume then has the rounding error of the other, and its NaN); of the middle (one CTA of 16 warps per SM: the plane
 // takes 148 KB) 0.6 ms are the depth sums.
 
 #include <algorithm>
@@ -384,7 +384,7 @@ __device__ __forceinline__ void rows_b(c32* sm, c32* S, const LineGeom& g, int n
     }
 }
 
-__global__ void __launch_bounds__(kRowsT, 3)
+__global__ void __launch_bounds__(kRowsT, 4)
 line_rows_kernel(const float* __restrict__ mu, const float2* __restrict__ Ty, c32* __restrict__ S,
                  LineGeom g) {
     extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
@@ -691,7 +691,7 @@ __device__ __forceinline__ void out_a(c32* sm, const LineGeom& g, const OutArgs&
     }
 }
 
-__global__ void __launch_bounds__(kRowsT, 3)
+__global__ void __launch_bounds__(kRowsT, 4)
 line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArgs o, LineGeom g) {
     extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
     const int P = g.y.n + 1;
