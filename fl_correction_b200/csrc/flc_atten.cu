@@ -531,7 +531,6 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
                      int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
                      int L, int a_base, int64_t out_a_stride, int64_t out_l_stride, void* workspace,
                      size_t ws_bytes, cudaStream_t st);
-bool cone_lines_first(int64_t Vn, int mode);
 int cone_fft_launch(const float* mu, const float* U, const float* Vw, float* out, int64_t Vn,
                     int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t My, int mode,
                     int L, int a_base, int64_t out_a_stride, int64_t out_l_stride,
@@ -577,19 +576,14 @@ int cone_launch_ws(const float* mu, const float* U, const float* Vw, float* out,
                    size_t ws_bytes, cudaStream_t st) {
     const int64_t var = tune(kTuneConeVariant);
     if (ws && (var == 0 || var == 4 || var == 5)) {
-        const bool lines = cone_lines_first(Vn, mode);
-        mode &= ~kConeWhole;
-        int r = FLC_ERR_UNSUPPORTED;
-        for (int k = 0; k < 2 && r == FLC_ERR_UNSUPPORTED; ++k)
-            r = (k == 0) == lines
-                    ? cone_line_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
-                                       out_a_stride, out_l_stride, ws, ws_bytes, st)
-                    : cone_fft_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
-                                      out_a_stride, out_l_stride, ws, ws_bytes, st);
+        int r = cone_line_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
+                                 out_a_stride, out_l_stride, ws, ws_bytes, st);
+        if (r == FLC_ERR_UNSUPPORTED)
+            r = cone_fft_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base,
+                                out_a_stride, out_l_stride, ws, ws_bytes, st);
         if (r != FLC_ERR_UNSUPPORTED) return r;
         clear_error();
     }
-    mode &= ~kConeWhole;
     return cone_sep_launch(mu, U, Vw, out, Vn, Z, X, Y, Mz, Mx, My, mode, L, a_base, out_a_stride,
                            out_l_stride, st);
 }
@@ -793,7 +787,7 @@ extern "C" int flc_cone_atten_separable(const float* mu, const float* u, const f
 extern "C" size_t flc_cone_atten_workspace_bytes(int64_t K, int64_t Z, int64_t X, int64_t Y,
                                                  int64_t Mz, int64_t Mx, int64_t My) {
     if (K < 1 || Z < 1 || X < 1 || Y < 1 || Mz < 1 || Mx < 1 || My < 1) return 0;
-    return cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, kConeWhole);
+    return cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
 }
 
 extern "C" int flc_cone_atten_separable_ws(const float* mu, const float* u, const float* v,
@@ -811,7 +805,7 @@ extern "C" int flc_cone_atten_separable_ws(const float* mu, const float* u, cons
         set_error("flc_cone_atten_separable_ws: workspace must be 256-byte aligned");
         return FLC_ERR_ALIGNMENT;
     }
-    return cone_launch_ws(mu, u, v, out, K, Z, X, Y, Mz, Mx, My, mode | kConeWhole, 1, 0, 0, 0, workspace,
+    return cone_launch_ws(mu, u, v, out, K, Z, X, Y, Mz, Mx, My, mode, 1, 0, 0, 0, workspace,
                           workspace ? workspace_bytes : 0, as_stream(stream));
 }
 
@@ -836,7 +830,7 @@ extern "C" int flc_cone_atten(const float* mu, const float* mask, float* out, in
         // where the shape takes it
         float* dbuf = nullptr;
         const size_t fbytes = align256(sizeof(float) * (U.size() + V.size()));
-        const size_t fft_bytes = cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, kConeWhole);
+        const size_t fft_bytes = cone_spec_ws_bytes(K, Z, X, Y, Mz, Mx, My, 0);
         const size_t bytes = fbytes + (fft_bytes ? fft_bytes + 256 : 0);
         FLC_TRY_CUDA(cudaMallocAsync((void**)&dbuf, bytes, st));
         int s = FLC_OK;
@@ -850,8 +844,8 @@ extern "C" int flc_cone_atten(const float* mu, const float* mask, float* out, in
             fft_ws = (void*)p;
         }
         if (s == FLC_OK)
-            s = cone_launch_ws(mu, dbuf, dbuf + U.size(), out, K, Z, X, Y, Mz, Mx, My, kConeWhole, 1, 0,
-                               0, 0, fft_ws, fft_bytes, st);
+            s = cone_launch_ws(mu, dbuf, dbuf + U.size(), out, K, Z, X, Y, Mz, Mx, My, 0, 1, 0, 0,
+                               0, fft_ws, fft_bytes, st);
         cudaFreeAsync(dbuf, st);
         // the host vectors are read by the copies above before they return
         cudaStreamSynchronize(st);

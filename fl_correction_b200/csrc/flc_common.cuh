@@ -81,8 +81,6 @@ int launch_cluster(const void* fn, dim3 grid, int G, size_t smem, cudaStream_t s
 // Bit of the cone `mode` argument that selects the plain separable kernel
 // over the TMA-pipelined one (for parity tests of both).
 constexpr int kConePlain = 0x100;
-// a call over given volumes, not part of a path that splits them (cone_lines_first)
-constexpr int kConeWhole = 0x200;
 
 // Device-side status left by bounded waits that gave up (flc_cone.cu).
 int cone_device_status(int reset);

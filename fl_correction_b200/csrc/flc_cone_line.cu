@@ -30,8 +30,12 @@
 // filter 0.01 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
 // the bytes they must at about half the copy rate, four CTAs an SM (three: 0.17 and 0.21;
 // two volumes as one complex one, with no half spectra to take apart, three CTAs: 0.15
-// and 0.20, but each volume then has the rounding error of the other, and its NaN); of the middle (one CTA of 16 warps per SM: the plane
-// takes 148 KB) 0.6 ms are the depth sums.
+// and 0.20, but each volume then has the rounding error of the other, and its NaN); of
+// the middle (one CTA of 16 warps per SM: the plane takes 148 KB) 0.6 ms are the depth
+// sums.  The line form is the faster one for few volumes too (planes / lines, us: 1
+// volume of 64^3 39 / 38, of 128^3 94 / 84, of 30 x 200^2 130 / 91; 2 of 48 x 64^2 42 /
+// 36, of 128^3 146 / 97; 3 of 96^3 101 / 87), so it runs wherever it takes the shape, and
+// a volume's bits do not depend on how many volumes are in the call.
 
 #include <algorithm>
 
@@ -803,19 +807,11 @@ size_t cone_line_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t M
     return line_ws(g, Vn, nullptr).bytes;
 }
 
-// The form tried first.  In a call over given volumes (kConeWhole), lines from four
-// on, planes below (us, planes / lines: 1 volume of 64^3 85 / 98, of 128^3 151 / 189; 2 of
-// 48 x 64^2 84 / 98, of 128^3 202 / 200; 3 of 96^3 151 / 162; 4 of 20 x 150^2 194 / 164,
-// of 128^3 320 / 255).  A path that goes over its volumes in parts takes lines whatever
-// the part, so that its results don't depend on the split.
-bool cone_lines_first(int64_t Vn, int mode) { return !(mode & kConeWhole) || Vn >= 4; }
-
 // Scratch bytes of the spectral cone, whichever form takes the shape.
 size_t cone_spec_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx,
                           int64_t My, int mode) {
     const size_t line = cone_line_ws_bytes(Vn, Z, X, Y, Mz, Mx, My);
-    const size_t plane = cone_fft_ws_bytes(Vn, Z, X, Y, Mz, Mx, My, mode & ~kConeWhole);
-    return line && (cone_lines_first(Vn, mode) || !plane) ? line : plane;
+    return line ? line : cone_fft_ws_bytes(Vn, Z, X, Y, Mz, Mx, My, mode);
 }
 
 // The path sum in the line form; arguments, modes and FLC_ERR_UNSUPPORTED as

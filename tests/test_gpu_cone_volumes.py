@@ -81,3 +81,12 @@ def test_lines_in_odd_chunks(chunk):
     full = XRFProjector(p, angles, mask, (S, N, N))
     part = XRFProjector(p, angles, mask, (S, N, N), chunk=chunk)
     assert torch.equal(full.project(T(frac)), part.project(T(frac)))
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_a_volume_alone_or_among_others(shape):
+    """A volume's bits, however many volumes the call holds."""
+    mu, mask = _case(*shape)
+    out = cal_atten_cuda(T(mu), T(mask))
+    for K in range(1, shape[0]):
+        assert torch.equal(cal_atten_cuda(T(mu[:K]), T(mask)), out[:K])
