@@ -762,29 +762,32 @@ bool line_geom(int64_t Z, int64_t X, int64_t Y, int64_t Mz, int64_t Mx, int64_t 
     return mid_smem(*g) <= cap && rows_smem(*g) <= cap;
 }
 
-// Volumes per pass: as many as fit in this much scratch.
+// Spectra held at a time: volumes are taken in batches of at most this much scratch.
 constexpr size_t kBatchBytes = 512u << 20;
 
 struct LineWs {
     double2 *Uf, *Vf;
     float2 *Tz, *Ty;
     c32 *G, *S;
-    int64_t batch;
+    int64_t batch;    // volumes whose spectra S holds
     size_t bytes;
 };
 
-LineWs line_ws(const LineGeom& g, int64_t Vn, char* base) {
+// The scratch that is asked for has room for min(Vn, the most of a batch) volumes, so a
+// call over fewer volumes never needs more; a call takes what it is given, `have` bytes,
+// for batches of one volume on (batch 0: not even that).
+LineWs line_ws(const LineGeom& g, int64_t Vn, char* base, size_t have) {
     LineWs w{};
     size_t off = 0;
     auto take = [&](size_t n) { char* p = base ? base + off : nullptr; off += al256(n); return p; };
     const size_t vol = sizeof(c32) * (size_t)g.Nyh * g.X * g.Z;
-    w.batch = std::max<int64_t>(1, std::min<int64_t>(Vn, (int64_t)(kBatchBytes / vol)));
-    w.batch = ceil_div(Vn, ceil_div(Vn, w.batch));                  // evened
     w.Uf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.z.n);
     w.Vf = (double2*)take(sizeof(double2) * (size_t)g.Mx * g.Nyh);
     w.Tz = (float2*)take(sizeof(float2) * g.z.n);
     w.Ty = (float2*)take(sizeof(float2) * g.y.n);
     w.G = (c32*)take(sizeof(c32) * (size_t)g.Nyh * std::min(g.Mx, g.X) * g.z.n);
+    w.batch = std::max<int64_t>(1, std::min<int64_t>(Vn, (int64_t)(kBatchBytes / vol)));
+    if (base) w.batch = have < off ? 0 : std::min<int64_t>(w.batch, (int64_t)((have - off) / vol));
     w.S = (c32*)take(vol * (size_t)w.batch);
     w.bytes = off;
     return w;
@@ -804,7 +807,7 @@ size_t cone_line_ws_bytes(int64_t Vn, int64_t Z, int64_t X, int64_t Y, int64_t M
                           int64_t My) {
     LineGeom g;
     if (tune(kTuneConeVariant) == 5 || !line_geom(Z, X, Y, Mz, Mx, My, &g)) return 0;
-    return line_ws(g, Vn, nullptr).bytes;
+    return line_ws(g, Vn, nullptr, 0).bytes;
 }
 
 // Scratch bytes of the spectral cone, whichever form takes the shape.
@@ -824,8 +827,8 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
     if (!workspace || Vn < 1 || Vn > 65535 || tune(kTuneConeVariant) == 5 ||
         !line_geom(Z, X, Y, Mz, Mx, My, &g) || ((uintptr_t)workspace & 255) != 0)
         return FLC_ERR_UNSUPPORTED;
-    const LineWs w = line_ws(g, Vn, (char*)workspace);
-    if (w.bytes > ws_bytes) return FLC_ERR_UNSUPPORTED;
+    const LineWs w = line_ws(g, Vn, (char*)workspace, ws_bytes);
+    if (w.batch < 1) return FLC_ERR_UNSUPPORTED;
     const size_t rsm = rows_smem(g), msm = mid_smem(g);
     FLC_TRY(allow_smem(line_rows_kernel, rsm));
     FLC_TRY(allow_smem(line_mid_kernel, msm));
@@ -838,9 +841,9 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
     FLC_TRY(check_launch("line_filter_kernel"));
     OutArgs o{out, mode, L, a_base, 0, out_a_stride, out_l_stride,
               (float)(0.5 / ((double)g.y.n * (double)g.z.n))};      // (line_rows leaves twice the spectra)
-    const int64_t vol = Z * X * Y;
-    for (int64_t v0 = 0; v0 < Vn; v0 += w.batch) {
-        const unsigned n = (unsigned)std::min<int64_t>(w.batch, Vn - v0);
+    const int64_t vol = Z * X * Y, batch = ceil_div(Vn, ceil_div(Vn, w.batch));   // evened
+    for (int64_t v0 = 0; v0 < Vn; v0 += batch) {
+        const unsigned n = (unsigned)std::min<int64_t>(batch, Vn - v0);
         line_rows_kernel<<<dim3((unsigned)ceil_div(Z, 2 * kLines), (unsigned)X, n), kRowsT, rsm, st>>>(
             mu + v0 * vol, w.Ty, w.S, g);
         FLC_TRY(check_launch("line_rows_kernel"));

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+from fl_correction_b200 import _lib, core
 from fl_correction_b200.cuda_lib import cal_atten_cuda
 from fl_correction_b200.xrf import XRFProjector
 from helpers import TOL_MAP, T
@@ -90,3 +91,66 @@ def test_a_volume_alone_or_among_others(shape):
     out = cal_atten_cuda(T(mu), T(mask))
     for K in range(1, shape[0]):
         assert torch.equal(cal_atten_cuda(T(mu[:K]), T(mask)), out[:K])
+
+
+def _spectral(mu, mask, nbytes):
+    """Path sums by flc_cone_atten_separable_ws with `nbytes` of scratch."""
+    K, Z, X, Y = mu.shape
+    u, v, (Mz, Mx, My) = core.mask_factors(mask, "cuda")
+    out = torch.full_like(mu, np.nan)
+    ws = _lib.workspace(nbytes, "cuda")
+    _lib.call("flc_cone_atten_separable_ws", _lib.ptr(mu), _lib.ptr(u), _lib.ptr(v), _lib.ptr(out), K, Z, X,
+              Y, Mz, Mx, My, 0, _lib.ptr(ws), nbytes, _lib.stream())
+    torch.cuda.synchronize()
+    return out
+
+
+def _bytes(K, shape):
+    return _lib.query("flc_cone_atten_workspace_bytes", K, *shape[1:])
+
+
+@pytest.mark.parametrize("shape", [(0, 128, 128, 128, 29, 128, 29), (0, 64, 256, 256, 59, 256, 59), SHAPES[0]])
+def test_fewer_volumes_need_no_more_scratch(shape):
+    n = [_bytes(K, shape) for K in range(1, 200)]
+    assert n[0] > 0 and n == sorted(n)
+
+
+def test_scratch_of_a_larger_call():
+    """55 volumes of 128^3 in the scratch of 144 (a last chunk of angles): the bits
+    of each volume alone."""
+    K, n = 55, 128
+    _, mask = _case(1, 1, 1, 1, 3, n, 5)
+    base = T(np.random.default_rng(1).random((1, n, n, n)))
+    scale = torch.rand((K, 1, 1, 1), device="cuda")
+    mu = base * scale
+    shape = (K, n, n, n) + mask.shape
+    out = _spectral(mu, mask, _bytes(144, shape))
+    for k in (0, 27, 28, K - 1):
+        assert torch.equal(_spectral(mu[k:k + 1], mask, _bytes(1, shape))[0], out[k])
+
+
+@pytest.mark.parametrize("held", [1, 2, 3])
+def test_volumes_in_batches(held):
+    """Scratch for fewer volumes than the call has: the same bits in several batches."""
+    mu, mask = _case(*SHAPES[0])
+    ref = _spectral(T(mu), mask, _bytes(5, SHAPES[0]))
+    assert torch.equal(_spectral(T(mu), mask, _bytes(held, SHAPES[0])), ref)
+
+
+def test_beam_layout_in_batches():
+    """exp(-res) multiplied into the attenuation, three angles of two lines in batches."""
+    rng = np.random.default_rng(4)
+    A, L, S, N = 3, 2, 6, 20
+    _, mask = _case(1, 1, 1, 1, 5, N, 5)
+    u, v, (Mz, Mx, My) = core.mask_factors(mask, "cuda")
+    mu = T(rng.random((A * L, S, N, N)))
+    outs = []
+    for held in (A * L, 4, 1):
+        out = T(np.ones((L, A, S, N, N)))
+        nb = _lib.query("flc_cone_fft_workspace_bytes", held, S, N, N, Mz, Mx, My)
+        ws = _lib.workspace(nb, "cuda")
+        _lib.call("flc_cone_atten_apply_ws", _lib.ptr(mu), _lib.ptr(u), _lib.ptr(v), _lib.ptr(out), A, L, S, N,
+                  N, A, 0, Mz, Mx, My, _lib.ptr(ws), nb, _lib.stream())
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
