@@ -111,8 +111,9 @@ few_frame_kernel(FewArgs P) {
             if (lane < 30 && m <= mhi && (unsigned)k < (unsigned)N && (low ? o < 0.f : o > edge) &&
                 (row || (x >= 0.f && x <= g.rmax)) && (w0 > 0.f || w1 > 0.f)) {
                 const float v = __ldg(at + h * N + w) * (rt ? __ldg(rt + w) : 1.f);
-                t0 = fmaf(w0, v, t0);
-                t1 = fmaf(w1, v, t1);
+                // (a value that is not finite stays with the positions it covers)
+                if (w0 > 0.f) t0 = fmaf(w0, v, t0);
+                if (w1 > 0.f) t1 = fmaf(w1, v, t1);
             }
         }
 #pragma unroll
@@ -143,7 +144,8 @@ few_frame_kernel(FewArgs P) {
 // Sum of atten * ratio * weight over the unclamped samples that cover pixel (i, j),
 // among the 3 x 3 around its inverse image.  EDGE: the pixel is within two of the
 // border, where samples in reach may be clamped (those are in the border sums; the
-// test is the forward's own).
+// test is the forward's own).  Attenuation and ratio count only where a sample covers
+// the pixel, also when they are not finite.
 template <bool EDGE>
 __device__ __forceinline__ float gather9(const Geo& g, const float* __restrict__ at,
                                          const float* __restrict__ rt, int N, float fi, float fj) {
@@ -165,6 +167,7 @@ __device__ __forceinline__ float gather9(const Geo& g, const float* __restrict__
         const bool win = (unsigned)(w0 + db) < (unsigned)N;
         const float wf = wr + (float)(db - 1) - g.cx;
         const float bx = fmaf(-g.s, wf, g.cy), by = fmaf(g.c, wf, g.cx);   // col_bx, col_by
+        bool any = false;
 #pragma unroll
         for (int da = 0; da < 3; ++da) {
             const float x = fmaf(g.c, hf[da], bx), y = fmaf(g.s, hf[da], by);
@@ -173,8 +176,9 @@ __device__ __forceinline__ float gather9(const Geo& g, const float* __restrict__
             if (EDGE) in = in && x >= 0.f && x <= g.rmax && y >= 0.f && y <= g.cmax;
             v[da][db] = in ? __ldg(p + da * N + db) : 0.f;
             wt[da][db] = wx * wy;
+            any = any || in;
         }
-        rr[db] = win ? (rt ? __ldg(rt + w0 + db) : 1.f) : 0.f;
+        rr[db] = any ? (rt ? __ldg(rt + w0 + db) : 1.f) : 0.f;
     }
 #pragma unroll
     for (int db = 0; db < 3; ++db) {
@@ -201,8 +205,10 @@ __device__ __noinline__ float gather_parts(float2 cs, const float* __restrict__ 
         const float hf = (float)h - g.cy;
         const float x = fmaf(g.c, hf, col_bx(g, w)), y = fmaf(g.s, hf, col_by(g, w));
         if (!(x >= 0.f && x <= g.rmax && y >= 0.f && y <= g.cmax)) continue;
+        const float cr = part_code(x, fi), cc = part_code(y, fj);
+        if (cr == 0.f || cc == 0.f) continue;
         const float v = __fmul_rn(__ldg(at + h * N + w), rt ? __fmul_rn(__ldg(rt + w), em) : em);
-        t += part_col(part_row(v, part_code(x, fi)), part_code(y, fj));
+        t += part_col(part_row(v, cr), cc);
     }
     return t;
 }
