@@ -105,10 +105,11 @@ class CorrectedMLEM:
         self.ws_mlem, self.ws_mlem_bytes = _lib.workspace_or_less(most, least, dev, free // (4 * n_ws))
         self._elem = None
         if self.concurrent and self.L > 1:
-            # one stream and one MLEM workspace per element
-            self._elem = [(torch.cuda.Stream(device=dev),
-                           self.ws_mlem if l == 0 else _lib.workspace(self.ws_mlem_bytes, dev))
-                          for l in range(self.L)]
+            # one stream and one MLEM workspace per element, each with its size (the
+            # copies where they can still be had)
+            ws = [(self.ws_mlem, self.ws_mlem_bytes)]
+            ws += [_lib.workspace_or_less(self.ws_mlem_bytes, least, dev) for _ in range(1, self.L)]
+            self._elem = [(torch.cuda.Stream(device=dev),) + w for w in ws]
 
     # -- building blocks -------------------------------------------------
     def recompute_attenuation(self, C, cone_events=None):
@@ -160,13 +161,13 @@ class CorrectedMLEM:
                 if mlem_events is not None:
                     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                     e0.record(main)
-                for l, (st, ws) in enumerate(self._elem):
+                for l, (st, ws, ws_bytes) in enumerate(self._elem):
                     st.wait_stream(main)
                     _lib.call("flc_mlem", _lib.ptr(C[l]), _lib.ptr(self.atten[l]),
                               _lib.ptr(self.em[l]), _lib.ptr(self.theta), _lib.ptr(I[l]),
                               int(n_iter), self.beta, self.delta, self.A, S, 1, H, W,
-                              _lib.ptr(ws), self.ws_mlem_bytes, 0, ctypes.c_void_p(st.cuda_stream))
-                for st, _ in self._elem:
+                              _lib.ptr(ws), ws_bytes, 0, ctypes.c_void_p(st.cuda_stream))
+                for st, _, _ in self._elem:
                     main.wait_stream(st)
                 if mlem_events is not None:
                     e1.record(main)
