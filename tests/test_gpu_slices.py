@@ -59,3 +59,25 @@ def test_angles_in_parts():
     ref = AC.backward_emission_batch(T(at), T(q), T(em), T(th))
     assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) < TOL_MAP
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("cluster", [1, 2])
+def test_more_angles_than_one_run_of_sums(cluster):
+    """70 angles in one or two CTAs of a tile: the register sums are put away every 32
+    angles, also after an angle on an axis."""
+    A, B, N = 70, 3, 20
+    rng = np.random.default_rng(cluster)
+    th = rng.uniform(-np.pi, np.pi, A)
+    th[[31, 34, 63, 69]] = [0.0, np.pi / 2, np.pi, -np.pi / 2]
+    at, C, em, th = projector_case(rng, A, B, 1, N, N, th)
+    q = rng.random((A, B, N)).astype(np.float32)
+    tune.set_knob("proj.cluster", cluster)
+    try:
+        out = AC.backward_emission_batch(T(at), T(q), T(em), T(th))
+        I = O.fwd_emission(at, C, em, th).astype(np.float32)
+        C0 = np.ones_like(C)
+        rec = AC.mlem_cuda_batch(T(C0), T(at), T(em), T(th), T(I), 2, 1e-3)
+    finally:
+        tune.set_knob("proj.cluster", 0)
+    assert rel_err(out.cpu().numpy(), O.bwd_emission(at, q, em, th)) < TOL_MAP
+    assert rel_err(rec.cpu().numpy(), O.mlem(C0, at, em, th, I, 2, 1e-3, 0.01)) < TOL_MLEM
