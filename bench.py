@@ -90,42 +90,31 @@ def mlem_bytes_per_iter(A, S, H, W, R=1):
     return fwd + bwd + upd
 
 
-# DRAM bytes measured by ncu with the kernels that these shapes took before the
-# line-form cone and the slice-lane projector: the plane form's five kernels move 54.3 MB
-# per 128^3 volume (325.8 MB read + write for 6 volumes); an MLEM iteration
-# at the benchmark's shape (120 angles x 128 slices of 128^2, one element)
-# moves 1.026 GB in the lean forward and 1.023 GB in the lean backward,
-# 1.018 bytes per attenuation byte.
-CONE_DRAM_BYTES_PER_VOLUME = 325.8e6 / 6
-MLEM_DRAM_PER_ATTEN_BYTE = (1.026144e9 + 1.023237e9) / (2 * 120 * 128 * 128 * 128 * 4)
+# DRAM bytes measured by ncu: the line form's kernels move 38.2 MB per 128^3 volume
+# (305.5 MB read + write for 8 volumes); an MLEM iteration at the benchmark's shape (120
+# angles x 128 slices of 128^2, one element) moves 1.066 GB in the slice-lane forward and
+# 0.929 + 0.137 GB in its backward and border sums, 1.059 bytes per attenuation byte.
+CONE_DRAM_BYTES_PER_VOLUME = 305.5e6 / 8
+MLEM_DRAM_PER_ATTEN_BYTE = (1.066248e9 + 0.928816e9 + 0.136750e9) / (2 * 120 * 128 * 128 * 128 * 4)
 # FP32 FMA rate measured on this pool's B200 (a chain-of-FMAs probe over
 # 148 x 8 CTAs of 256 threads)
 FP32_PEAK_TFLOPS = 72.5
 
 
-def smooth_even(n):
-    """Smallest even m >= n whose only prime factors are 2, 3 and 5 (the
-    spectral cone's transform lengths)."""
-    m = n + (n & 1)
-    while True:
-        k = m
-        for r in (2, 3, 5):
-            while k % r == 0:
-                k //= r
-        if k == 1:
-            return m
-        m += 2
+# transform lengths of the spectral cone's line form
+LINE_LENGTHS = (16, 24, 32, 40, 48, 54, 64, 72, 80, 90, 96, 108, 120, 128, 144, 160, 180, 192, 216,
+                240, 256, 288, 320, 400)
 
 
 def spectral_cone_flops(Z, X, Y, Mz, Mx, My):
-    """FLOPs of the spectral cone for one volume: the depth correlation
+    """FLOPs of the spectral cone's line form for one volume: the depth sums
     (8 per complex multiply-add, every frequency of every target plane and
     depth inside the volume) and the 2-D transforms (5 N log2 N per complex
     transform of length N; rows in pairs, then the half-spectrum columns),
     forward and inverse."""
     hz, hy = Mz // 2, My // 2
-    Nz = smooth_even(Z + max(1, hz, Mz - 1 - hz))
-    Ny = smooth_even(Y + max(hy, My - 1 - hy))
+    Nz = next(n for n in LINE_LENGTHS if n >= Z + max(hz, Mz - 1 - hz))
+    Ny = next(n for n in LINE_LENGTHS if n >= Y + max(hy, My - 1 - hy))
     Nyh = Ny // 2 + 1
     pairs = sum(min(Mx, X - x) for x in range(X))
     corr = 8.0 * Nz * Nyh * pairs
@@ -320,6 +309,8 @@ def run_ours(args, rank, world, device):
     value = job_rate(world, n_iter * args.steps, ms_max)
     e2e_value = job_rate(world, n_iter * args.steps, e2e_ms)
     cone_share = t_cone / ms if ms else 0.0
+    # whether the solver's MLEM holds the slice-lane copies
+    lanes = solver.ws_mlem_bytes > _lib.query("flc_mlem_workspace_bytes", A, N, 1, N, N)
     line = {
         "metric": METRIC,
         "value": round(value, 3),
@@ -350,14 +341,14 @@ def run_ours(args, rank, world, device):
         # the dominant kernel: the fused MLEM iteration (with the sensitivity
         # backward of each attenuation rebuild)
         "roofline": {
-            "kernel": "MLEM iteration: slices_fwd_kernel (+ ratio), slices_frame_kernel and slices_bwd_kernel (+ update), "
-                      "with the sensitivity backward of each rebuild", "bound": "hbm",
+            "kernel": ("MLEM iteration: slices_fwd_kernel (+ ratio), slices_frame_kernel and slices_bwd_kernel (+ update)"
+                       if lanes else "MLEM iteration: projector kernels of flc_project.cu or flc_few.cu")
+                      + ", with the sensitivity backward of each rebuild", "bound": "hbm",
             "achieved": round(proj_gbs, 1) if proj_gbs else None, "peak": hbm, "unit": "GB/s",
             "frac": round(proj_gbs / hbm, 3) if proj_gbs else None,
-            "traffic": round(MLEM_DRAM_PER_ATTEN_BYTE * 2 * A * N ** 3 * 4),
-            "traffic_note": "per element-iteration: ncu dram read + write of the splat forward and backward "
-                            "(proj_fwd2, proj_bwd2) at this shape; the slice-lane pair reads the attenuation "
-                            "twice as well, not captured",
+            "traffic": round(MLEM_DRAM_PER_ATTEN_BYTE * 2 * A * N ** 3 * 4) if lanes else None,
+            "traffic_note": "per element-iteration: ncu dram read + write of the slice-lane forward, border sums and "
+                            "backward at 120 angles x 128 slices of 128^2, scaled by the attenuation's bytes",
             "peak_kind": peak_kind,
             "algorithmic_unit": "%.4g B per element-iteration (fwd + bwd + update at the reference API "
                                 "boundary) and %.4g B per sensitivity pass (one per element and "
@@ -371,9 +362,9 @@ def run_ours(args, rank, world, device):
             "unit": "TFLOP/s",
             "frac": round(spec * vols_per_launch / (cone_avg_ms * 1e-3) / 1e12 / fp32_peak, 3),
             "traffic": round(CONE_DRAM_BYTES_PER_VOLUME * vols_per_launch * (N / 128) ** 3),
-            "traffic_note": "ncu dram read+write of the plane form's kernels on 6 volumes of 128^3, per volume, times volumes per launch; the line form not captured",
+            "traffic_note": "ncu dram read + write of these kernels on 8 volumes of 128^3, per volume, times volumes per launch",
             "peak_kind": "measured FP32 FMA rate (chain-of-FMAs probe on this pool's B200)",
-            "algorithmic_unit": "spectral FLOPs of the plane form (direct depth correlation + 2-D FFTs, %dx%d padded planes) = %.3g per volume; the line form does fewer"
+            "algorithmic_unit": "FLOPs of the line form (direct depth sums + 2-D FFTs, %dx%d padded planes) = %.3g per volume"
                                 % (nz_ny[0], nz_ny[1], spec),
             "launches": cone_launches, "avg_ms": round(cone_avg_ms, 4),
             "separable_equivalent_tflops": round(2 * sep * vols_per_launch / (cone_avg_ms * 1e-3) / 1e12, 1),

@@ -52,8 +52,9 @@ enum TuneKey {
                             // bands only slices that do not fit in shared memory)
     kTuneProjSlices = 10,   // slice-lane kernels where scratch is given: 0 automatic,
                             // 1 wherever they take the shape, 2 never
-    kTuneProjFew = 11,      // gather backward for few slices where scratch is given:
-                            // 0 automatic, 1 wherever it takes the shape, 2 never
+    kTuneProjFew = 11,      // gather kernels for few slices (the backward where scratch
+                            // is given, every forward): 0 automatic, 1 wherever they
+                            // take the shape, 2 never
     kTuneCount = 12
 };
 int64_t tune(int key);

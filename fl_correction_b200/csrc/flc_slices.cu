@@ -20,9 +20,9 @@
 //             registers: no atomics, no phases, no barriers.
 //
 // 120 angles x 128 slices of 128^2 (1 GB of attenuation, 0.15 ms at the measured
-// copy rate): copy 0.31 ms, forward 0.23 ms (lean kernel 0.42), backward 0.47 ms
-// (lean kernel 1.37); flc_mlem with 5 iterations 4.3 ms (10.4).  180 angles x 32
-// slices of 256^2: forward 0.62 ms (2.71), backward 1.48 ms (4.96 in row bands).
+// copy rate): copy 0.31 ms, forward 0.23 ms (lean kernel 0.42), backward 0.42 + 0.08 ms
+// (lean kernel 1.37); flc_mlem with 5 iterations 4.4 ms (10.3).  180 angles x 32
+// slices of 256^2: forward 0.63 ms (2.71), backward 1.37 + 0.17 ms (4.96 in row bands).
 //
 // Reference semantics as in flc_project.cu (atten_cuda_kernel.cu:91-446).
 
@@ -202,9 +202,9 @@ slices_out_kernel(const float* __restrict__ src, float* __restrict__ dst, int B,
 // ---------------------------------------------------------------------------
 // Forward: grid (ceil(N / 8), A, slice groups); warp = detector column.  The
 // lanes work out the weights of 32 samples of the column at a time.  out =
-// em * sum, or I / max(that, 1e-6) when I != nullptr.  Bound by the attenuation
-// it streams (1.0 GB in 0.23 ms, 4.4 TB/s); the eight columns of a CTA walk the
-// beam side by side, so the taps of one are mostly in L1 from another.
+// em * sum, or I / max(that, 1e-6) when I != nullptr.  Bound by the L1 (71% busy) and the
+// latency of the attenuation it streams (1.05 GB in 0.23 ms, 4.5 TB/s); the eight columns
+// of a CTA walk the beam side by side, so the taps of one are mostly in L1 from another.
 // ---------------------------------------------------------------------------
 constexpr int kFU = 4;     // samples whose loads are issued together
 
@@ -306,6 +306,7 @@ slices_fwd_kernel(const float* __restrict__ at, const float* __restrict__ C,
 constexpr int kSlots = 16;       // list entries per block of 2 x 2 pixels (the open square of
                                  // side 3 that they cover holds at most 13 lattice points, or
                                  // 4 x 4 where it is aligned to within rounding)
+constexpr int kAlways = 10;      // entries that are always added, without branches
 constexpr int kSub = 4;          // lanes that build one list together
 constexpr int kFlush = 32;       // angles summed in registers before they are added to the
                                  // tile's image: short sums, for their rounding error
@@ -357,7 +358,7 @@ struct SArgs {
 // the 5 x 5 around the block's inverse image, with their weights (times
 // `scale`) for the four pixels, position and column.  kSub adjacent lanes take
 // the candidates in turn.  Sample points are computed by the forward's
-// expressions.  A list is filled up to eight entries, and to an even number,
+// expressions.  A list is filled up to kAlways entries, and to an even number,
 // with its first sample at weight 0.  Returns the number of samples.
 __device__ __forceinline__ int list_samples(const Geo& g, int N, float i, float j, float scale,
                                             bool live, int lane, float4* wl, uint2* ol) {
@@ -397,7 +398,7 @@ __device__ __forceinline__ int list_samples(const Geo& g, int N, float i, float 
     __syncwarp();
     if (n > 0 || !live) {
         const uint2 f = live ? ol[0] : make_uint2(0u, 0u);
-        const int upto = n <= 10 ? 10 : (n + 1) & ~1;
+        const int upto = n <= kAlways ? kAlways : (n + 1) & ~1;
         for (int e = n + sub; e < upto; e += kSub) {
             wl[e] = make_float4(0.f, 0.f, 0.f, 0.f);
             ol[e] = f;
@@ -607,8 +608,9 @@ __device__ __noinline__ float covered_sum(const float* __restrict__ at, const fl
 
 // The backward: unclamped samples, then the border sums.  Grid (G * tiles, slice
 // groups), cluster (G, 1, 1): CTA g of a tile sums angles [g * apc, ...).
-// Bound by the latency and the L1 wavefronts of its loads (two 128 NS byte runs,
-// attenuation and ratio, per sample and block of pixels).  What brought the 120
+// Bound by the latency of its loads (two 128 NS byte runs, attenuation and ratio, per
+// sample and block of pixels; 16 warps an SM issue in 37% of the slots and wait for these,
+// the L1 is 44% busy, and each byte comes from HBM once).  What brought the 120
 // angles x 128 slices of 128^2 down: one pixel at a time, the list's loads behind
 // a branch per pixel 0.68 ms (NS = 4; 1.33 and 2.75 ms with NS = 2 and 1); loads
 // of several pixels in flight 0.59; blocks of 2 x 2 pixels, nine samples instead
@@ -699,7 +701,7 @@ slices_bwd_kernel(SArgs P) {
         const int l0 = (warp * NA + par) * BPW;
         const float4* wl = swl + l0 * L::WP;
         const uint2* ol = sol + l0 * L::OP;
-        // the first eight of every block, without branches so that many loads
+        // the first kAlways of every block, without branches so that many loads
         // are in flight; a block that no sample reaches (outside the rotated
         // slice) has no list
         if (near_axis(g, N)) {
@@ -716,20 +718,22 @@ slices_bwd_kernel(SArgs P) {
         if (some == kAll) {
 #pragma unroll
             for (int k = 0; k < BPW; ++k) {
-                add_block<NS, RATIO, 5>(ab, rb, pitch, wl + k * L::WP + 0, ol + k * L::OP + 0, acc[k]);
-                add_block<NS, RATIO, 5>(ab, rb, pitch, wl + k * L::WP + 5, ol + k * L::OP + 5, acc[k]);
+                add_block<NS, RATIO, kAlways / 2>(ab, rb, pitch, wl + k * L::WP, ol + k * L::OP, acc[k]);
+                add_block<NS, RATIO, kAlways / 2>(ab, rb, pitch, wl + k * L::WP + kAlways / 2,
+                                                  ol + k * L::OP + kAlways / 2, acc[k]);
             }
         } else {
 #pragma unroll
             for (int k = 0; k < BPW; ++k) {
                 if (!(some >> k & 1u)) continue;
-                add_block<NS, RATIO, 5>(ab, rb, pitch, wl + k * L::WP + 0, ol + k * L::OP + 0, acc[k]);
-                add_block<NS, RATIO, 5>(ab, rb, pitch, wl + k * L::WP + 5, ol + k * L::OP + 5, acc[k]);
+                add_block<NS, RATIO, kAlways / 2>(ab, rb, pitch, wl + k * L::WP, ol + k * L::OP, acc[k]);
+                add_block<NS, RATIO, kAlways / 2>(ab, rb, pitch, wl + k * L::WP + kAlways / 2,
+                                                  ol + k * L::OP + kAlways / 2, acc[k]);
             }
         }
 #pragma unroll
         for (int k = 0; k < BPW; ++k)
-            for (int e = 10; e < cnts[k]; e += 2)
+            for (int e = kAlways; e < cnts[k]; e += 2)
                 add_block<NS, RATIO, 2>(ab, rb, pitch, wl + k * L::WP + e, ol + k * L::OP + e, acc[k]);
         if ((a - a0) % kFlush == kFlush - 1) flush();
     }
@@ -839,15 +843,18 @@ bool slices_takes(int64_t A, int64_t B, int64_t H, int64_t W) {
 
 // Whether a call that has the scratch goes to the slice-lane kernels (the
 // "proj.slices" knob: 1 wherever they take the shape, 2 never).  A group of 32
-// slices costs the same however many of them exist, and the copies and the
-// five launches of a backward have to be paid for; measured in microseconds,
-// lean or band kernels / these:
-//   MLEM, 5 iterations: 60 angles 64^2 x 16 slices 608 / 596, 90 x 96^2: 24 slices
-//   1371 / 1223, 33 1473 / 1588, 48 1823 / 1595; 120 x 128^2: 8 slices 2701 /
-//   2529, 128 10373 / 4239; 180 x 256^2: 8 14316 / 12297, 32 43533 / 12258.
-//   One backward: 120 x 128^2: 16 slices 465 / 433, 128 1373 / 866; 96^2: 48
-//   236 / 283, 96 414 / 364; 64^2: 48 106 / 109, 64 124 / 114; 30 x 48^2: 64
-//   53 / 71, 128 91 / 76; 256^2: 8 1839 / 2312, 32 4990 / 2336.
+// slices costs the same however many of them exist (33 to 37 are padded to 64, which
+// below 112^2 the splats still beat), and the copies and the five launches of a backward
+// have to be paid for.  Up to ten slices the kernels of flc_few.cu are the others, above
+// the lean or band kernels.  Microseconds, others / these:
+//   MLEM, 5 iterations: 60 angles 64^2 x 16 slices 617 / 598; 90 x 96^2: 8 899 / 1252,
+//   24 1368 / 1245, 33 1478 / 1624, 48 1821 / 1619; 120 x 128^2: 8 1743 / 2599, 12
+//   2896 / 2600 (the one side of the line where the other would be a little faster), 16
+//   3202 / 2597, 128 10341 / 4440; 180 x 256^2: 8 8991 / 12963, 32 36790 / 12944.
+//   One backward: 120 x 128^2: 8 slices 245 / 430, 16 463 / 432, 128 1369 / 903; 90 x
+//   96^2: 48 234 / 286, 96 411 / 378; 60 x 64^2: 48 104 / 110, 64 123 / 115; 30 x 48^2:
+//   64 51 / 69, 128 90 / 79 (by the line at 8 million samples 64 stay with the others);
+//   180 x 256^2: 8 1202 / 2344, 16 2764 / 2346, 32 4986 / 2379.
 bool use_slices(int64_t A, int64_t B, int64_t H, int64_t W, bool mlem) {
     const int64_t knob = tune(kTuneProjSlices);
     if (tune(kTuneProjLegacy) != 0 || tune(kTuneProjBand) != 0 || knob == 2) return false;

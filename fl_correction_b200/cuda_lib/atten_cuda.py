@@ -105,7 +105,8 @@ def forward_emission_batch(atten, C, em_cs, theta):
 
 def backward_emission_batch(atten, ratio, em_cs, theta):
     """out (R,B,H,W), the exact transpose of forward_emission_batch applied to
-    ratio (A,B,W) (atten_cuda.cpp:188-214)."""
+    ratio (A,B,W) (atten_cuda.cpp:188-214).  For volumes the call holds copies of
+    about 512 MB of atten at a time (one angle's at least)."""
     _lib.require_cuda("backward_emission_batch", atten, ratio, em_cs, theta)
     if atten.dim() != 4 or ratio.dim() != 3 or em_cs.dim() != 2 or theta.dim() != 1:
         raise RuntimeError("backward_emission_batch: expects atten (A,B,H,W), ratio (A,B,W), "
@@ -159,7 +160,9 @@ def huber_grad(C, grad, delta):
 
 def mlem_cuda_batch(C_init, atten, em_cs, theta, I, n_iter, beta=1e-3, delta=0.01):
     """MLEM with optional Huber term (atten_cuda.cpp:283-345): returns a new
-    (R,B,H,W) tensor; C_init is not modified."""
+    (R,B,H,W) tensor; C_init is not modified.  For the length of the call the
+    slice-lane kernels hold a second copy of atten, its slices rounded up to 32,
+    64 or 128 (where that is at most a quarter of the device's memory)."""
     _lib.require_cuda("mlem_cuda_batch", C_init, atten, em_cs, theta, I)
     if C_init.dim() != 4 or atten.dim() != 4 or I.dim() != 3:
         raise RuntimeError("mlem_cuda_batch: C_init (R,B,H,W), atten (A,B,H,W), I (A,B,W)")

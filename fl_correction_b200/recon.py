@@ -43,6 +43,11 @@ class CorrectedMLEM:
                    quantile; threshold mask 1).  'bounded' keeps cal_frac's
                    non-negativity and replaces its quantile clamp and
                    percentile scaling by the mass-fraction bound.
+
+    The object keeps the attenuation (L, A, S, N, N) and, where the slice-lane
+    kernels take the shape, one more copy of it for the MLEM: all elements' (one
+    element's without `concurrent`) where these take at most a quarter of the
+    memory that is free when the object is made, none otherwise.
     """
 
     def __init__(self, param, angles_deg, mask, shape, fixed_frac=None, incident="own",

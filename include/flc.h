@@ -78,10 +78,11 @@ FLC_API uint64_t flc_launch_count(void);
  *                   slice, or the fewest even bands that fit in shared memory)
  *   "proj.slices"   the slice-lane kernels of flc_mlem and flc_bwd_emission_ws (square
  *                   slices, where scratch is given): 1 wherever they take the shape, 2
- *                   never; automatic: from 16 slices on
- *   "proj.few"      the gather backward for few slices of flc_mlem and
- *                   flc_bwd_emission_ws (square slices): 1 wherever it takes the shape,
- *                   2 never
+ *                   never; automatic: flc_mlem from 16 slices on, flc_bwd_emission_ws from
+ *                   16 slices of 128^2 or 64 of fewer pixels on, past a number of samples
+ *   "proj.few"      the gather kernels for few slices: the backward of flc_mlem and
+ *                   flc_bwd_emission_ws (square slices) and the forward of every entry
+ *                   point that has one: 1 wherever they take the shape, 2 never
  * Test hooks of the direct cone's bounded waits (for failure-path tests):
  *   "cone.test_wait_limit"  polls before a TMA-plane wait gives up (default 2^26)
  *   "cone.test_skip_load"   k > 0: the load of the k-th staged plane of every
@@ -127,7 +128,11 @@ FLC_API int flc_cone_atten_separable(const float* mu, const float* u, const floa
  * factorisation and scratch allocation): `workspace` (256-byte aligned) of
  * flc_cone_atten_workspace_bytes(K, Z, X, Y, Mz, Mx, My) bytes; where that is
  * 0 (the padded planes do not fit) or workspace is NULL, the direct separable
- * kernel runs.  mode 0 writes the sum, 1 exp(-sum).  Same results as
+ * kernel runs.  The bytes never decrease with K, and a workspace for fewer
+ * volumes serves a call over more (in batches, with the same results) where the
+ * line form takes the shape.  A volume's sum depends on that volume alone, a
+ * plane's on the planes from it to the detector, whatever else the call holds.
+ * mode 0 writes the sum, 1 exp(-sum).  Same results as
  * flc_cone_atten to FP32 rounding.  Counterpart: cal_atten_cuda
  * (atten_cuda.cpp:12-28) with the mask factored once by the caller. */
 FLC_API size_t flc_cone_atten_workspace_bytes(int64_t K, int64_t Z, int64_t X, int64_t Y,
@@ -158,8 +163,11 @@ FLC_API int flc_bwd_emission(const float* atten, const float* ratio, const float
 /* flc_bwd_emission with caller scratch, for volumes: `workspace` (256-byte
  * aligned) of flc_bwd_emission_workspace_bytes(...) bytes lets the backward
  * run on slice-fastest copies of a part of the angles at a time (about 512
- * MB), with the slices as lanes.  Where that is 0 (few slices, slices that are
- * not square), or workspace is NULL or smaller, the call is flc_bwd_emission. */
+ * MB), with the slices as lanes, or for few slices in the gather kernels, whose
+ * border sums it holds.  Where that is 0 (slices that are not square, numbers of
+ * slices between the two), or workspace is NULL or smaller, the call is
+ * flc_bwd_emission.  A value that is not finite reaches the pixels whose bilinear
+ * footprint it lies in. */
 FLC_API size_t flc_bwd_emission_workspace_bytes(int64_t A, int64_t B, int64_t R, int64_t H,
                                                 int64_t W);
 FLC_API int flc_bwd_emission_ws(const float* atten, const float* ratio, const float* em,
@@ -180,7 +188,8 @@ FLC_API int flc_huber_grad(const float* C, float* grad, int64_t RB, int64_t H, i
  * copies C_init first, as the reference's clone does).  I is (A,B,W).
  * The caller provides `workspace` of at least flc_mlem_workspace_bytes(...)
  * bytes (256-byte aligned).  With use_graph != 0 the iteration is captured
- * once into a CUDA graph and replayed n_iter times.  A workspace of
+ * once into a CUDA graph and replayed n_iter times (ignored where the slice-lane
+ * kernels or those for few slices run, which are launched plainly).  A workspace of
  * flc_mlem_workspace_bytes_ex(...) bytes lets volumes of one reference run on
  * slice-fastest copies of the attenuation, the projections and the images,
  * with the slices as lanes (it holds a copy of the attenuation; where that
