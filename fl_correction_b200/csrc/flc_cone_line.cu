@@ -615,6 +615,14 @@ line_mid_kernel(c32* __restrict__ S, const c32* __restrict__ G, const float2* __
 // Rows inverse: grid (ceil(X / 32), ceil(Z / 2), volumes).  Slices z and z + 1 (if it
 // exists) are the real and the imaginary part.
 // ---------------------------------------------------------------------------
+// Where the results go: the reference layout; the beam layout; the beam layout, multiplying
+// an attenuation that is loaded before the last DFTs.  The loads ahead take registers, three
+// CTAs an SM instead of four; they pay up to DFTs of kAheadR points (us, ahead / not: 36
+// volumes of 128^3, 12 points, 243 / 442; 24 of 96^3, 12, 89 / 163; 40 of 61 x 111^2, 16,
+// 262 / 185; 12 of 150^3, 18, 401 / 322).
+enum { kRef, kBeam, kBeamAhead };
+constexpr int kAheadR = 12;
+
 struct OutArgs {
     float* out;
     int mode;                // 0 res, 1 exp(-res) in the reference layout;
@@ -655,7 +663,7 @@ __device__ __forceinline__ void out_b(const c32* S, c32* sm, const float2* tw, c
     }
 }
 
-template <int R, int R2>
+template <int R, int R2, int TO>
 __device__ __forceinline__ void out_a(c32* sm, const LineGeom& g, const OutArgs& o, float* oa, float* ob,
                                       int nl) {
     constexpr int r2 = R2, P = R * R2 + 1;
@@ -664,8 +672,10 @@ __device__ __forceinline__ void out_a(c32* sm, const LineGeom& g, const OutArgs&
     for (int n2 = threadIdx.x >> 5; n2 < r2; n2 += kRowsT / 32) {
         c32 v[R];
         float pa[R], pb[R];
-        if (R <= 16 && o.mode == 2) {
-            // the attenuation of these pixels, loaded before the last DFTs
+        constexpr bool ahead = TO == kBeamAhead && R <= kAheadR;
+        // (the mode is known to be 2: the branch keeps the loads from being moved down
+        // to their use, 243 against 352 us)
+        if (ahead && o.mode == 2) {
 #pragma unroll
             for (int n1 = 0; n1 < R; ++n1) {
                 const int y = r2 * n1 + n2;
@@ -683,19 +693,20 @@ __device__ __forceinline__ void out_a(c32* sm, const LineGeom& g, const OutArgs&
             un(v[n1], ra, rb);
             ra *= o.scale;
             rb *= o.scale;
-            if (o.mode < 2) {
+            if constexpr (TO == kRef) {
                 sm[l * P + y] = mk(o.mode ? expf(-ra) : ra, o.mode ? expf(-rb) : rb);
             } else if (y < g.Y) {
                 const int64_t at = (int64_t)(g.Y - 1 - y) * g.X + l;
                 const float ea = expf(-ra), eb = expf(-rb);
-                oa[at] = o.mode == 2 ? (R <= 16 ? pa[n1] : oa[at]) * ea : ea;
-                if (ob) ob[at] = o.mode == 2 ? (R <= 16 ? pb[n1] : ob[at]) * eb : eb;
+                oa[at] = o.mode == 2 ? (ahead ? pa[n1] : oa[at]) * ea : ea;
+                if (ob) ob[at] = o.mode == 2 ? (ahead ? pb[n1] : ob[at]) * eb : eb;
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(kRowsT, 4)
+template <int TO>
+__global__ void __launch_bounds__(kRowsT, TO == kBeamAhead ? 3 : 4)
 line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArgs o, LineGeom g) {
     extern __shared__ __align__(16) c32 sm[];                       // [32][Ny + 1], twiddles
     const int P = g.y.n + 1;
@@ -712,17 +723,17 @@ line_out_kernel(const c32* __restrict__ S, const float2* __restrict__ Ty, OutArg
     __syncthreads();
     const int v = o.v0 + blockIdx.z;
     float* oa;
-    if (o.mode >= 2) {
+    if constexpr (TO != kRef) {
         const int al = v / o.L, l = v - al * o.L;
         oa = o.out + l * o.l_stride + (int64_t)(o.a_base + al) * o.a_stride + (int64_t)z * g.Y * g.X + x0;
     } else {
         oa = o.out + (((int64_t)v * g.Z + z) * g.X + x0) * g.Y;
     }
     float* ob = two ? oa + (int64_t)g.X * g.Y : nullptr;
-#define CALL(A, B) out_a<A, B>(sm, g, o, oa, ob, nl)
+#define CALL(A, B) out_a<A, B, TO>(sm, g, o, oa, ob, nl)
     FLC_LEN(g.y)
 #undef CALL
-    if (o.mode >= 2) return;
+    if constexpr (TO != kRef) return;
     __syncthreads();
     const float rY = 1.f / (float)g.Y;
     for (int i = threadIdx.x; i < nl * g.Y; i += kRowsT) {
@@ -832,7 +843,10 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
     const size_t rsm = rows_smem(g), msm = mid_smem(g);
     FLC_TRY(allow_smem(line_rows_kernel, rsm));
     FLC_TRY(allow_smem(line_mid_kernel, msm));
-    FLC_TRY(allow_smem(line_out_kernel, rsm));
+    const auto out_kernel = mode < 2 ? line_out_kernel<kRef>
+                            : mode == 2 && g.y.r1 <= kAheadR ? line_out_kernel<kBeamAhead>
+                                                             : line_out_kernel<kBeam>;
+    FLC_TRY(allow_smem(out_kernel, rsm));
     line_roots_kernel<<<(unsigned)g.Mx + 1, 256, sizeof(double2) * (size_t)(g.z.n + g.y.n), st>>>(
         U, Vw, w.Uf, w.Vf, w.Tz, w.Ty, g);
     FLC_TRY(check_launch("line_roots_kernel"));
@@ -850,7 +864,7 @@ int cone_line_launch(const float* mu, const float* U, const float* Vw, float* ou
         line_mid_kernel<<<dim3((unsigned)g.Nyh, n), kMidT, msm, st>>>(w.S, w.G, w.Tz, g);
         FLC_TRY(check_launch("line_mid_kernel"));
         o.v0 = (int)v0;
-        line_out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)ceil_div(Z, 2), n), kRowsT, rsm, st>>>(
+        out_kernel<<<dim3((unsigned)ceil_div(X, kLines), (unsigned)ceil_div(Z, 2), n), kRowsT, rsm, st>>>(
             w.S, w.Ty, o, g);
         FLC_TRY(check_launch("line_out_kernel"));
     }
