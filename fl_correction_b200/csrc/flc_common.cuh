@@ -68,6 +68,10 @@ int smem_per_sm();
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// Whether the lean splats' slice image (R references, rows padded) is small enough for
+// three CTAs an SM, where they are at their best: R = 1 up to 128^2, 3 up to 64^2.
+inline bool small_image(int64_t R, int64_t H, int64_t W) { return 4 * R * H * (W + 9) <= 72 * 1024; }
+
 // Cluster launches over the angles of a projector kernel (flc_project.cu).
 struct ClusterPlan {
     int G;      // CTAs per slice or tile (cluster size)

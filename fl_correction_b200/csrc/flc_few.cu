@@ -358,12 +358,18 @@ int few_splits(int64_t A, int64_t B, int64_t N) {
 // 141 for 10, 163 / 165 for 12; 120 of 128^2 405 / 233 for 8; 40 of 24^2 40 / 33 for 10.
 // Two references: 75 of 33 x 101^2 512 / 429, but 30 of 31 x 64^2 89 / 97; past 128^2
 // the splats take one reference at a time: 60 of 64 x 192^2 4216 / 1984.  Three: 120 of
-// 33 x 101^2 1512 / 657, 60 of 31 x 48^2 155 / 109, 30 of 200 x 16^2 101 / 88.
+// 33 x 101^2 1512 / 657, 60 of 31 x 48^2 155 / 109; where the splats run with three CTAs
+// an SM (small_image) they are ahead again from some slices on: 40 of 24^2: 33 slices 74 /
+// 50, 70 79 / 87, 150 104 / 164; 60 of 48^2: 33 150 / 143, 70 184 / 280; 60 of 64^2: 33 212 /
+// 221; MLEM of 60 x 48^2, 5 iterations: 70 1606 / 2207, 150 3709 / 4770; five references: 40
+// of 24^2: 30 97 / 52, 100 109 / 136; 60 of 48^2: 30 213 / 155, 100 399 / 464.
 bool use_few(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W) {
     const int64_t knob = tune(kTuneProjFew);
     if (tune(kTuneProjLegacy) != 0 || tune(kTuneProjBand) != 0 || knob == 2) return false;
     if (H != W || H < 16 || R > kFewR || B > 65535 || H * W > (1 << 30)) return false;
-    return knob == 1 || B <= (R == 1 ? 10 : 26) || R > 2 || (R == 2 && W > 128);
+    if (knob == 1) return true;
+    if (R > 2) return !small_image(R, H, W) || B * W < 400 * R + 400;
+    return B <= (R == 1 ? 10 : 26) || (R == 2 && W > 128);
 }
 
 int64_t few_floats(int64_t A, int64_t B, int64_t R, int64_t N) {

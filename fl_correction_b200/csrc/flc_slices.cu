@@ -855,14 +855,22 @@ bool slices_takes(int64_t A, int64_t B, int64_t H, int64_t W) {
 //   96^2: 48 234 / 286, 96 411 / 378; 60 x 64^2: 48 104 / 110, 64 123 / 115; 30 x 48^2:
 //   64 51 / 69, 128 90 / 79 (by the line at 8 million samples 64 stay with the others);
 //   180 x 256^2: 8 1202 / 2344, 16 2764 / 2346, 32 4986 / 2379.
-bool use_slices(int64_t A, int64_t B, int64_t H, int64_t W, bool mlem) {
+// Where the lean splats run with three CTAs an SM (small_image), a backward whose slices
+// fill their group badly, or with few angles, loses: 60 x 64^2: 72 slices (of 128) 130 /
+// 157, 136 (of 192) 214 / 252, 96 171 / 158; 40 x 80^2: 65 110 / 168; 90 x 96^2: 72 305 /
+// 370, 136 506 / 758, 96 410 / 372; 40 x 128^2: 16 154 / 175, 48 198 / 224, 72 302 / 332,
+// 96 365 / 334; 120 x 128^2: 33 481 / 529, 40 548 / 531, 65 717 / 889, 96 1047 / 891; two
+// references, 60 x 64^2: 70 230 / 265, 100 333 / 264.
+bool use_slices(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W, bool mlem) {
     const int64_t knob = tune(kTuneProjSlices);
     if (tune(kTuneProjLegacy) != 0 || tune(kTuneProjBand) != 0 || knob == 2) return false;
     if (!slices_takes(A, B, H, W)) return false;
     if (knob == 1) return true;
     const int64_t work = A * B * H * W;
     if (mlem) return B >= 16 && work >= 3000000 && !(H < 112 && B > 32 && B < 38);
-    return B >= (H >= 128 ? 16 : 64) && work >= 8000000;
+    if (B < (H >= 128 ? 16 : 64) || work < 8000000) return false;
+    if (!small_image(R, H, W)) return true;
+    return B > 64 ? 4 * B >= 3 * slices_pad(B) : A >= 48 && (B <= 32 || B >= 40);
 }
 
 int slices_in(const float* src, float* dst, int64_t n, int64_t B, int64_t M, cudaStream_t st) {
@@ -974,7 +982,7 @@ size_t bwd_bytes(int64_t A, int64_t R, int64_t N, int64_t Bp) {
 
 // Scratch of mlem_slices, 0 where it does not take the call.
 size_t mlem_slices_bytes(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W) {
-    if (R != 1 || !use_slices(A, B, H, W, true)) return 0;
+    if (R != 1 || !use_slices(A, B, R, H, W, true)) return 0;
     return mlem_bufs(A, H, slices_pad(B), nullptr).bytes;
 }
 
@@ -1027,7 +1035,7 @@ using namespace flc;
 extern "C" size_t flc_bwd_emission_workspace_bytes(int64_t A, int64_t B, int64_t R, int64_t H,
                                                    int64_t W) {
     if (A < 1 || B < 1 || R < 1 || H < 2 || W < 2) return 0;
-    if (use_slices(A, B, H, W, false)) return bwd_bytes(A, R, H, slices_pad(B));
+    if (use_slices(A, B, R, H, W, false)) return bwd_bytes(A, R, H, slices_pad(B));
     return use_few(A, B, R, H, W) ? sizeof(float) * (size_t)few_floats(A, B, R, H) : 0;
 }
 
@@ -1044,7 +1052,7 @@ extern "C" int flc_bwd_emission_ws(const float* atten, const float* ratio, const
     }
     const size_t need = flc_bwd_emission_workspace_bytes(A, B, R, H, W);
     if (workspace && need && workspace_bytes >= need) {
-        if (use_slices(A, B, H, W, false))
+        if (use_slices(A, B, R, H, W, false))
             return bwd_slices(atten, ratio, em, theta, out, A, B, R, H, workspace, as_stream(stream));
         return bwd_few_launch(atten, ratio, em, theta, out, nullptr, nullptr, (float*)workspace, A, B, R, H,
                               0.f, 0, 0.f, 0.f, as_stream(stream));
