@@ -21,6 +21,8 @@ namespace flc {
 
 // Whether the lean forward takes the slice (flc_project.cu).
 bool fwd2_takes(int64_t R, int64_t H, int64_t W);
+// ... and whether it is compiled for the width.
+bool fwd2_fixed_width(int64_t W);
 
 namespace {
 
@@ -385,7 +387,16 @@ bool use_few_fwd(int64_t A, int64_t B, int64_t R, int64_t H, int64_t W) {
     // with 2 references 48.5 / 35.4 for 4, 227 / 258 for 33.  Where it does not, the
     // first forward, us: 180 of 256^2 141 / 51 for 1 slice, 2694 / 1346 for 32; 60 of
     // 512^2 554 / 73 for 1)
-    return knob == 1 || B <= (R == 1 ? 2 : 8) || !fwd2_takes(R, H, W);
+    if (knob == 1 || !fwd2_takes(R, H, W)) return true;
+    // (tall slices have few columns to share out: 60 of 200 x 64, 1 and 2 slices, 24 / 21
+    // and 21 / 27, with two references 34 / 31 and 35 / 50)
+    if (H > 2 * W) return B == 1;
+    if (R == 1) return B <= 2;
+    // (up to 128^2 the lean forward is at its best at its compile-time widths: two
+    // references, 60 of 64^2: 2 slices 21 / 21, 6 20 / 25, 8 21 / 29, 120 of 128^2: 4 86 / 79, 6
+    // 100 / 111, 8 129 / 144; at others 60 of 101^2: 6 52 / 42, 8 53 / 54; above, 30 of 160^2:
+    // 8 107 / 69)
+    return B <= (H * W > 128 * 128 || !fwd2_fixed_width(W) ? 8 : small_image(R, H, W) ? 2 : 4);
 }
 
 // Forward: out (A, B, W) = P C, or I / max(P C, 1e-6) when I != nullptr.

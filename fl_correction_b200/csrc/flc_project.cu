@@ -1686,6 +1686,8 @@ bool fwd2_takes(int64_t R, int64_t H, int64_t W) {
     return fwd2_smem(R, H, W) <= (size_t)max_smem_optin();
 }
 
+bool fwd2_fixed_width(int64_t W) { return fwd2_for_width<1>(W) != fwd2_for_width<1>(0); }
+
 // Lean forward (+ ratio when I != nullptr); FLC_ERR_UNSUPPORTED (nothing
 // launched) when the slice does not fit in shared memory.
 int fwd2_launch(const float* atten, const float* C, const float* em, const float* theta,
