@@ -26,7 +26,7 @@
 //                 writes exp(-res) into the beam layout (x is its fastest axis,
 //                 so no transpose is left) or res into the reference layout
 //
-// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.16, middle 0.85, out 0.18,
+// 36 volumes of 128^3 with a 29 x 128 x 29 mask: rows 0.16, middle 0.86, out 0.18,
 // filter 0.01 ms, against 2.2 ms in five kernels of the plane form.  Rows and out move
 // the bytes they must at about half the copy rate, four CTAs an SM (three: 0.17 and 0.21;
 // two volumes as one complex one, with no half spectra to take apart, three CTAs: 0.15
@@ -489,12 +489,12 @@ __device__ __forceinline__ void mid_zo(const c32* pl, c32* S, const LineGeom& g,
 // ones, so what a round writes nobody reads any more.  Middle kernel, 36 volumes of 128^3:
 // tiles of 12 planes 1.00 ms, 10 0.94, 8 0.82, 6 0.89 (four warps a scheduler, and what
 // the registers leave for loads in flight; 768 threads of 80 registers 1.06); the sums cut
-// at 64 depths and G four steps ahead instead of eight 0.85 (two steps 0.86, eight 0.92,
-// the depths in halves on two lanes 0.94).
+// at 32 depths and G four steps ahead instead of eight 0.86 (cut at 64 0.85, with G two steps
+// ahead 0.86, eight 0.92; the depths in halves on two lanes 0.94).
 // ---------------------------------------------------------------------------
 constexpr int kTile = 8;
 constexpr int kAhead = 4;        // steps that G is loaded ahead of its use
-constexpr int kRun = 64;         // depths summed in one go: short sums, for their rounding error
+constexpr int kRun = 32;         // depths summed in one go: short sums, for their rounding error
 
 struct DepthSum {
     c32 p[kTile], q[kTile], w[kTile], gv[kAhead], sum[kTile];
