@@ -353,12 +353,10 @@ int few_splits(int64_t A, int64_t B, int64_t N) {
 // Whether a backward of these sizes goes to the gather kernels for few slices, with
 // few_floats(...) floats of scratch (the "proj.few" knob: 1 wherever they take the
 // shape, 2 never).  Their time goes with the slices, the splats' has a floor; more
-// references cost the splats in proportion and these next to nothing.  The line is drawn
-// by the slice count alone, so some larger calls of two references stay with the splats
-// although these would be faster (33 x 101^2 below).  One backward
+// references cost the splats in proportion and these next to nothing.  One backward
 // with its allocation, us, splats / these: 90 angles of 96^2 161 / 36 for 1 slice, 163 /
 // 141 for 10, 163 / 165 for 12; 120 of 128^2 405 / 233 for 8; 40 of 24^2 40 / 33 for 10.
-// Two references: 75 of 33 x 101^2 512 / 429, but 30 of 31 x 64^2 89 / 97; past 128^2
+// Two references: 75 of 33 x 101^2 512 / 510, 30 of 31 x 64^2 89 / 97; past 128^2
 // the splats take one reference at a time: 60 of 64 x 192^2 4216 / 1984.  Three: 120 of
 // 33 x 101^2 1512 / 657, 60 of 31 x 48^2 155 / 109; where the splats run with three CTAs
 // an SM (small_image) they are ahead again from some slices on: 40 of 24^2: 33 slices 74 /
